@@ -176,11 +176,9 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   c->cnt2 = dalloc<uint32_t>(cfg->n, "cnt2");
   check_cuda(cudaMemset(c->cnt1, 0, cfg->m * 4), "cnt1");
   check_cuda(cudaMemset(c->cnt2, 0, cfg->n * 4), "cnt2");
-  if (cfg->exec == DSGDPP_EXEC_HOGWILD) {
-    const size_t cs = cfg->precision == kFp64 ? 8 : 4;
-    check_cuda(cudaMalloc(&c->inv1, cfg->m * cs), "inv1");
-    check_cuda(cudaMalloc(&c->inv2, cfg->n * cs), "inv2");
-  }
+  const size_t cs = cfg->precision == kFp64 ? 8 : 4;
+  check_cuda(cudaMalloc(&c->inv1, cfg->m * cs), "inv1");
+  check_cuda(cudaMalloc(&c->inv2, cfg->n * cs), "inv2");
   c->h_schedule = halloc<uint32_t>((size_t)d2 * d, "schedule");
   c->d_schedule = dalloc<uint32_t>((size_t)d2 * d, "schedule");
   c->h_params = halloc<EpochParams>(1, "params");
@@ -295,6 +293,15 @@ void reserve_records(DevMatrix& M, uint64_t u, bool as_double) {
   M.col = dalloc<uint32_t>(u, "col");
   check_cuda(cudaMalloc(&M.val, u * (as_double ? 8 : 4)), "val");
   M.cap = u;
+}
+
+// The update weights 1 / nnz1 and 1 / nnz2 of the counts in place.  The replay
+// divides as the reference does (a count of 0 gives infinity).
+void inverse_counts(dsgdpp_ctx* c, cudaStream_t st) {
+  const bool as_double = c->cfg.precision == kFp64;
+  const bool of_zero = c->cfg.exec == DSGDPP_EXEC_REPLAY;
+  check_cuda(launch_inverse_counts(c->cnt1, c->cfg.m, c->inv1, as_double, of_zero, st), "inv1");
+  check_cuda(launch_inverse_counts(c->cnt2, c->cfg.n, c->inv2, as_double, of_zero, st), "inv2");
 }
 
 // Fills the device input arrays (rows, cols, values) of the blocking: the
@@ -493,10 +500,7 @@ void set_matrix_impl(dsgdpp_ctx* c, int which, uint64_t nnz, const uint32_t* row
     check_cuda(cudaMemsetAsync(c->cnt1, 0, c->cfg.m * 4, st), "cnt1");
     check_cuda(cudaMemsetAsync(c->cnt2, 0, c->cfg.n * 4, st), "cnt2");
     check_cuda(launch_count_nnz12(M.row, M.col, u, c->cnt1, c->cnt2, st), "nnz12");
-    if (c->inv1) {
-      check_cuda(launch_inverse_counts(c->cnt1, c->cfg.m, c->inv1, as_double, st), "inv1");
-      check_cuda(launch_inverse_counts(c->cnt2, c->cfg.n, c->inv2, as_double, st), "inv2");
-    }
+    inverse_counts(c, st);
   }
   if (vals_on_side) check_cuda(cudaStreamWaitEvent(st, c->ev_vals, 0), "wait values");
   check_cuda(launch_gather_values(perm, u, head_at, skeys, sidx, nnz, t_vals, M.val, as_double,
@@ -776,7 +780,7 @@ void run_replay_epoch(dsgdpp_ctx* c, double eps, const uint32_t* seeds, uint32_t
   }
   ReplayArgs a{};
   a.row = M.row; a.col = M.col; a.val = static_cast<const double*>(M.val);
-  a.cnt1 = c->cnt1; a.cnt2 = c->cnt2;
+  a.inv1 = static_cast<const double*>(c->inv1); a.inv2 = static_cast<const double*>(c->inv2);
   a.W = static_cast<double*>(c->W); a.H = static_cast<double*>(c->H);
   a.block_ptr = M.block_ptr; a.schedule = c->d_schedule;
   a.positions = c->d_positions; a.pos_offset = c->d_pos_offset; a.params = c->d_params;
@@ -1085,11 +1089,7 @@ int dsgdpp_set_counts(dsgdpp_ctx* c, const uint64_t* nnz1, const uint64_t* nnz2)
     check_cuda(cudaMemcpyAsync(d + m, nnz2, n * 8, cudaMemcpyHostToDevice, st), "H2D nnz2");
     check_cuda(launch_counts_to_u32(d, m, c->cnt1, st), "nnz1");
     check_cuda(launch_counts_to_u32(d + m, n, c->cnt2, st), "nnz2");
-    if (c->inv1) {
-      const bool as_double = c->cfg.precision == kFp64;
-      check_cuda(launch_inverse_counts(c->cnt1, m, c->inv1, as_double, st), "inv1");
-      check_cuda(launch_inverse_counts(c->cnt2, n, c->inv2, as_double, st), "inv2");
-    }
+    inverse_counts(c, st);
     check_cuda(cudaStreamSynchronize(st), "sync");
     return DSGDPP_OK;
   });

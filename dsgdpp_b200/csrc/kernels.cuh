@@ -45,14 +45,14 @@ struct HogwildArgs {
   double lambda, tmin, tmax;
 };
 
-// Deterministic FP64 replay: one warp per task walks its block in the
-// host-generated point order; d blocks of a sub-epoch run side by side.
+// Deterministic FP64 replay: one CTA per task runs its block with the results
+// of the host-generated point order; d blocks of a sub-epoch run side by side.
 struct ReplayArgs {
   const uint32_t* row;
   const uint32_t* col;
   const double* val;
-  const uint32_t* cnt1;  // nnz1 per row
-  const uint32_t* cnt2;  // nnz2 per column
+  const double* inv1;    // 1 / nnz1 per row
+  const double* inv2;    // 1 / nnz2 per column
   double* W;
   double* H;
   const uint64_t* block_ptr;  // d*nb2+1
@@ -250,8 +250,8 @@ cudaError_t launch_counts_to_u32(const uint64_t* in, uint64_t len, uint32_t* out
                                  cudaStream_t st);
 cudaError_t launch_count_nnz12(const uint32_t* row, const uint32_t* col, uint64_t nnz,
                                uint32_t* cnt1, uint32_t* cnt2, cudaStream_t st);
-cudaError_t launch_inverse_counts(const uint32_t* cnt, uint64_t len, void* inv,
-                                  int as_double, cudaStream_t st);
+cudaError_t launch_inverse_counts(const uint32_t* cnt, uint64_t len, void* inv, int as_double,
+                                  int of_zero, cudaStream_t st);
 cudaError_t launch_factor_to_device(int precision, const double* src, uint64_t rows,
                                     uint32_t r, uint32_t rp, void* dst, cudaStream_t st);
 cudaError_t launch_factor_to_host(int precision, const void* src, uint64_t rows, uint32_t r,

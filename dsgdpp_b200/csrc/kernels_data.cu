@@ -215,12 +215,15 @@ __global__ void count_nnz12_kernel(const uint32_t* row, const uint32_t* col, uin
   }
 }
 
-__global__ void inverse_counts_kernel(const uint32_t* cnt, uint64_t len, void* inv, int as_double) {
+// 1 / count; of a count of 0: 0, or 1 / 0 with of_zero
+__global__ void inverse_counts_kernel(const uint32_t* cnt, uint64_t len, void* inv, int as_double,
+                                      int of_zero) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < len; k += stride) {
     const uint32_t c = cnt[k];
-    if (as_double) reinterpret_cast<double*>(inv)[k] = c ? 1.0 / (double)c : 0.0;
-    else reinterpret_cast<float*>(inv)[k] = c ? 1.0f / (float)c : 0.0f;
+    const bool div = c != 0 || of_zero;
+    if (as_double) reinterpret_cast<double*>(inv)[k] = div ? __ddiv_rn(1.0, (double)c) : 0.0;
+    else reinterpret_cast<float*>(inv)[k] = div ? 1.0f / (float)c : 0.0f;
   }
 }
 
@@ -358,9 +361,9 @@ cudaError_t launch_count_nnz12(const uint32_t* row, const uint32_t* col, uint64_
 }
 
 cudaError_t launch_inverse_counts(const uint32_t* cnt, uint64_t len, void* inv, int as_double,
-                                  cudaStream_t st) {
+                                  int of_zero, cudaStream_t st) {
   if (len == 0) return cudaSuccess;
-  inverse_counts_kernel<<<kGrid, 256, 0, st>>>(cnt, len, inv, as_double);
+  inverse_counts_kernel<<<kGrid, 256, 0, st>>>(cnt, len, inv, as_double, of_zero);
   return cudaGetLastError();
 }
 

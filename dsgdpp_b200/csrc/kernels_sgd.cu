@@ -10,10 +10,13 @@
 //    every SM draws 32-record chunks from.  Inside a warp, groups of LPN lanes
 //    each own one record; a lane moves VPL 16-byte vectors of the W row and of
 //    the H column.  Within a block updates run concurrently (Hogwild).
-//  * replay_subepoch: the deterministic FP64 mode.  One warp per task walks its
-//    block in the exact point order of the reference and repeats every
-//    floating-point operation of the reference in the same order, without FMA
-//    contraction, so the result matches the CPU restatement bit for bit.
+//  * replay_subepoch: the deterministic FP64 mode.  One CTA per task runs its
+//    block with the results of the reference's exact point order, records
+//    without a common row or column together, and repeats every floating-point
+//    operation of the reference in the same order, without FMA contraction, so
+//    the result matches the CPU restatement bit for bit.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace dsgdpp {
@@ -712,171 +715,295 @@ __global__ void build_segments_kernel(SegBuildArgs a) {
 }
 
 // ---- deterministic FP64 replay ---------------------------------------------
-constexpr int kReplayMaxK = 8;  // r <= 256
+// One CTA per task.  The reference updates a block's records one after the
+// other; two records that share neither their row of W nor their column of H
+// commute exactly, so a record may run as soon as every earlier record on its
+// row or column has run, and every update still reads the values the
+// sequential order gives it.  The CTA keeps K = 512 / G records in hand, one
+// per group of G lanes, and works in rounds of one barrier each:
+//  * every record in hand has posted its place in the order at a slot of its
+//    row and a slot of its column (shared memory, minimum wins);
+//  * a record that finds its own place at both slots runs: no earlier record
+//    in hand has its row or column, and the earlier records that are not in
+//    hand are done.  Two rows that share a slot only delay the later record;
+//  * while its rows are loaded, its group takes the next record of the order
+//    and every record that will be in hand posts for the next round.
+// The earliest record in hand always runs, so every round makes progress.
+// Posts of a round go to the table of its parity (the other one is being
+// read), stamped with the round so that what an older round left is larger
+// and the tables need no clearing.  Coordinates, values and inverse counts
+// come through a ring in shared memory, loaded some rounds ahead in three
+// steps (position -> coordinates and value -> inverse counts).
+//
+// Bound: the latency of a round -- a barrier, the slots, the rows, the serial
+// z-order sum -- over the records that run in it: almost K where rows and
+// columns rarely repeat, down to one where a block is mostly one column.
+// Measured per epoch against one warp walking each task's records in order:
+// 1M uniform entries, rank 10, d = 4: 294 -> 4.4 ms; rank 32, d = 8: 232 ->
+// 4.1 ms; 500k Zipf(1.1) entries, rank 10, d = 16: 60 -> 34 ms; rank 128,
+// d = 8: 455 -> 67 ms.  With the rows loaded before the slots are known and
+// two barriers a round: 4.7 and 36 ms.
+constexpr int kReplayThreads = 512;
+constexpr uint32_t kReplaySlotBits = 11;
+constexpr uint32_t kReplaySlots = 1u << kReplaySlotBits;  // per side and parity
+constexpr uint32_t kReplayRoundBits = 11;  // of a post: rounds left, then the place
+constexpr uint32_t kReplayPlaceBits = 32 - kReplayRoundBits;
 
-__global__ void __launch_bounds__(128) replay_subepoch_kernel(ReplayArgs a, uint32_t s) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (id >= a.d) return;
-  const uint32_t d = a.d, r = a.r;
-  const uint32_t b2 = a.schedule[(size_t)s * d + id];
-  const uint64_t blk = (uint64_t)id * a.nb2 + b2;
+struct ReplayRec {
+  uint32_t i, j;
+  double x, f3, f4;  // value, 1 / nnz1[i], 1 / nnz2[j]
+};
+
+template <int G>
+constexpr size_t replay_smem() {
+  return sizeof(ReplayRec) * 8 * (kReplayThreads / G) + 4 * sizeof(uint32_t) * kReplaySlots;
+}
+
+// G lanes per record, KP elements of each row per lane (as KP / 2 vectors:
+// element e of vector v of lane l is z = 2 (l + G v) + e); r <= G * KP.
+template <int G, int KP>
+__global__ void __launch_bounds__(kReplayThreads, 1)
+    replay_subepoch_kernel(ReplayArgs a, uint32_t s) {
+  constexpr uint32_t K = kReplayThreads / G, CAP = 8 * K;
+  constexpr int NV = KP / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ReplayRec* ring = reinterpret_cast<ReplayRec*>(smem_raw);
+  uint32_t* slots = reinterpret_cast<uint32_t*>(ring + CAP);  // [parity][side][slot]
+  __shared__ uint32_t s_asked[3];  // records asked for in this round, the last, the next
+
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, gl = tid % G, id = blockIdx.x;
+  const uint32_t d = a.d, r = a.r, rp = a.rp;
+  const uint64_t blk = (uint64_t)id * a.nb2 + a.schedule[(size_t)s * d + id];
   const uint64_t rb = a.block_ptr[blk];
-  const uint64_t n = a.block_ptr[blk + 1] - rb;
+  const uint32_t n = (uint32_t)(a.block_ptr[blk + 1] - rb);
+  if (n == 0) return;
   const uint32_t* pos = a.positions + a.pos_offset[(size_t)s * d + id];
   const double eps = a.params->eps;
-  const int kmax = (int)((r + 31) / 32);
   // f1 = eps * -2. * (x - wh); f2 = eps * 2. * lambda
   const double em2 = __dmul_rn(eps, -2.0);
   const double f2 = __dmul_rn(__dmul_rn(eps, 2.0), a.lambda);
-
-  if (n == 0) return;
-  // The reads run ahead of the updates: the coordinates, value and counts of
-  // record q + 2 and the factor rows of record q + 1 are loaded while record q
-  // is updated.  Record q + 1 takes a row or column that record q writes from
-  // q's new values in registers (each lane reads back only the elements it
-  // writes itself, so rows written earlier are seen in program order); every
-  // update therefore reads the values the sequential order gives it, and the
-  // arithmetic below is the reference's, operation for operation.
-  struct Coord {
-    uint32_t i, j, c1, c2;
-    double x;
-  };
   const bool counts = a.update == kUpdNzslL2;
-  auto load_coord = [&](uint64_t q) {
-    Coord e;
-    const uint64_t rec = rb + pos[q];
-    e.i = a.row[rec];
-    e.j = a.col[rec];
-    e.x = a.val[rec];
-    e.c1 = counts ? a.cnt1[e.i] : 1u;
-    e.c2 = counts ? a.cnt2[e.j] : 1u;
-    return e;
-  };
-  auto load_rows = [&](const Coord& e, double (&wz)[kReplayMaxK], double (&hz)[kReplayMaxK]) {
-    const double* w = a.W + (size_t)e.i * a.rp;
-    const double* h = a.H + (size_t)e.j * a.rp;
-#pragma unroll
-    for (int k = 0; k < kReplayMaxK; ++k) {
-      const uint32_t z = (uint32_t)k * 32 + lane;
-      wz[k] = 0;
-      hz[k] = 0;
-      if (k < kmax && z < r) {
-        wz[k] = w[z];
-        hz[k] = h[z];
-      }
-    }
-  };
-  Coord cur = load_coord(0);
-  Coord nxt = n > 1 ? load_coord(1) : cur;
-  double wz[kReplayMaxK], hz[kReplayMaxK];
-  load_rows(cur, wz, hz);
 
-#pragma unroll 1
-  for (uint64_t q = 0; q < n; ++q) {
-    const Coord after = q + 2 < n ? load_coord(q + 2) : nxt;
-    double nwz[kReplayMaxK], nhz[kReplayMaxK];
-    if (q + 1 < n) load_rows(nxt, nwz, nhz);
-    double pz[kReplayMaxK];
+  for (uint32_t k = tid; k < 4 * kReplaySlots; k += kReplayThreads) slots[k] = 0xffffffffu;
+  if (tid < 3) s_asked[tid] = 0;
+
+  // the loads ahead: threads 0 .. K-1 each bring one record per round
+  uint32_t fetch = 0;                                      // next record to bring
+  uint32_t ready1 = 0, ready2 = 0, ready3 = 0, ready = 0;  // brought so far, by step; in the ring
+  uint32_t q1 = 0, q2 = 0, q3 = 0, p1 = 0;                 // place and position by step
+  bool v1 = false, v2 = false, v3 = false;
+  ReplayRec e2{}, e3{};
+
+  bool have = false;  // a record in hand: its place, its post, itself
+  uint32_t q = 0, post = 0, row_at = 0, col_at = 0;
+  ReplayRec e{};
+  uint32_t taken = 0, limit = 0;  // records handed out; those that could be last round
+  uint32_t rounds_left = (1u << kReplayRoundBits) - 1, base = 0, par = 0, now3 = 0;
+  for (;;) {
+    // everything written and posted last round is visible
+    if (!__syncthreads_or(have ? 1 : 0) && taken == n) break;
+    taken = min(taken + s_asked[now3 == 0 ? 2 : now3 - 1], limit);
+    if (tid == 0) s_asked[now3 == 2 ? 0 : now3 + 1] = 0;
+    limit = ready;
+
+    // 1. the records that come first on their row and column run
+    const bool go = have && slots[row_at] == post && slots[col_at] == post;
+    const bool any_go = __any_sync(kFullMask, go);
+    double* w = a.W + (size_t)e.i * rp;
+    double* h = a.H + (size_t)e.j * rp;
+    const double x = e.x, f3 = e.f3, f4 = e.f4;
+    double wz[KP], hz[KP];
 #pragma unroll
-    for (int k = 0; k < kReplayMaxK; ++k) {
-      const uint32_t z = (uint32_t)k * 32 + lane;
-      pz[k] = (k < kmax && z < r) ? __dmul_rn(wz[k], hz[k]) : 0.0;
+    for (int v = 0; v < NV; ++v) {
+      const uint32_t z = 2 * (gl + G * v);
+      double2 tw = make_double2(0, 0), th = make_double2(0, 0);
+      if (go && z < rp) {
+        tw = *reinterpret_cast<const double2*>(w + z);
+        th = *reinterpret_cast<const double2*>(h + z);
+      }
+      wz[2 * v] = tw.x;
+      wz[2 * v + 1] = tw.y;
+      hz[2 * v] = th.x;
+      hz[2 * v + 1] = th.y;
     }
-    // wh = sum_z w[z] h[z] in z order (every lane computes the same sum)
-    double wh = 0;
-#pragma unroll
-    for (int k = 0; k < kReplayMaxK; ++k) {
-      if (k >= kmax) break;
-      for (uint32_t l = 0; l < 32; ++l) {
-        if ((uint32_t)k * 32 + l >= r) break;
-        wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[k], l));
+
+    // 2. while they travel: groups that are or will be free take the next records
+    have = have && !go;
+    const uint32_t want = __ballot_sync(kFullMask, !have && gl == 0);
+    if (want) {
+      uint32_t first = 0;
+      if (lane == 0) first = atomicAdd(&s_asked[now3], (uint32_t)__popc(want));
+      first = taken + __shfl_sync(kFullMask, first, 0);
+      if (!have) {
+        q = first + __popc(want & ((1u << (lane - gl)) - 1u));
+        have = q < limit;
+        if (have) e = ring[q % CAP];
       }
     }
-    const double f1 = __dmul_rn(em2, __dsub_rn(cur.x, wh));
-    double f3 = 0, f4 = 0;
-    if (counts) {
-      f3 = __ddiv_rn(1.0, (double)cur.c1);
-      f4 = __ddiv_rn(1.0, (double)cur.c2);
+    par ^= 1u;
+    now3 = now3 == 2 ? 0 : now3 + 1;
+    if (--rounds_left == 0) {
+      // all round numbers used: places count from a new base.  A record in
+      // hand waits for at most K others, of which one runs per round while at
+      // most K are handed out, so its place is within K^2 <= 2^18 of the last
+      // one handed out; what is handed out stays below base + 2^19 + 2^11 K,
+      // within the place bits.
+      rounds_left = (1u << kReplayRoundBits) - 1;
+      base = taken > (1u << 19) ? taken - (1u << 19) : 0;
+      __syncthreads();  // every group has read its slots
+      for (uint32_t k = tid; k < 4 * kReplaySlots; k += kReplayThreads) slots[k] = 0xffffffffu;
+      __syncthreads();
     }
-    double* w = a.W + (size_t)cur.i * a.rp;
-    double* h = a.H + (size_t)cur.j * a.rp;
-#pragma unroll
-    for (int k = 0; k < kReplayMaxK; ++k) {
-      const uint32_t z = (uint32_t)k * 32 + lane;
-      if (k >= kmax || z >= r) continue;
-      const double t = wz[k];
-      double nw, nh;
-      if (a.update == kUpdNzsl) {
-        nw = __dsub_rn(wz[k], __dmul_rn(f1, hz[k]));
-        nh = __dsub_rn(hz[k], __dmul_rn(f1, t));
-      } else if (a.update == kUpdNzslL2) {
-        nw = __dsub_rn(wz[k], __dadd_rn(__dmul_rn(f1, hz[k]), __dmul_rn(__dmul_rn(f2, wz[k]), f3)));
-        nh = __dsub_rn(hz[k], __dadd_rn(__dmul_rn(f1, t), __dmul_rn(__dmul_rn(f2, hz[k]), f4)));
-      } else {
-        nw = __dsub_rn(wz[k], __dadd_rn(__dmul_rn(f1, hz[k]), __dmul_rn(f2, wz[k])));
-        nh = __dsub_rn(hz[k], __dadd_rn(__dmul_rn(f1, t), __dmul_rn(f2, hz[k])));
-      }
-      if (a.truncate) {
-        if (nw <= a.tmin) nw = __dadd_rn(a.tmin, eps);
-        else if (nw >= a.tmax) nw = __dsub_rn(a.tmax, eps);
-        if (nh <= a.tmin) nh = __dadd_rn(a.tmin, eps);
-        else if (nh >= a.tmax) nh = __dsub_rn(a.tmax, eps);
-      }
-      w[z] = nw;
-      h[z] = nh;
-      // record q + 1 on the same row or column reads these values
-      if (nxt.i == cur.i) nwz[k] = nw;
-      if (nxt.j == cur.j) nhz[k] = nh;
+    post = rounds_left << kReplayPlaceBits | (q - base);
+    row_at = par * 2 * kReplaySlots + ((e.i * 0x9E3779B1u) >> (32 - kReplaySlotBits));
+    col_at = par * 2 * kReplaySlots + kReplaySlots + ((e.j * 0x9E3779B1u) >> (32 - kReplaySlotBits));
+    if (have && gl == 0) {
+      // a post that is not the minimum so far is left out: of the many records
+      // that wait for a hot column only the first few queue at its slot
+      volatile uint32_t* sl = slots;
+      if (post < sl[row_at]) atomicMin(slots + row_at, post);
+      if (post < sl[col_at]) atomicMin(slots + col_at, post);
     }
-    __syncwarp();
-    if (q + 1 == n) break;
-    cur = nxt;
-    nxt = after;
+
+    // 3. the loads ahead: each step on what the step before it loaded last round
+    if (tid < K) {
+      if (v3) ring[q3 % CAP] = e3;
+      v3 = v2;
+      q3 = q2;
+      e3.i = e2.i;
+      e3.j = e2.j;
+      e3.x = e2.x;
+      if (v3 && counts) {
+        e3.f3 = a.inv1[e2.i];
+        e3.f4 = a.inv2[e2.j];
+      }
+      v2 = v1;
+      q2 = q1;
+      if (v2) {
+        const uint64_t rec = rb + p1;
+        e2.i = a.row[rec];
+        e2.j = a.col[rec];
+        e2.x = a.val[rec];
+      }
+    }
+    ready = ready3;
+    ready3 = ready2;
+    ready2 = ready1;
+    const uint32_t cnt = min(min(K, n - fetch), CAP - (fetch - taken));
+    v1 = tid < cnt;
+    q1 = fetch + tid;
+    if (v1) p1 = pos[q1];
+    fetch += cnt;
+    ready1 = fetch;
+
+    // 4. the update
+    if (any_go) {
+      double pz[KP];
 #pragma unroll
-    for (int k = 0; k < kReplayMaxK; ++k) {
-      wz[k] = nwz[k];
-      hz[k] = nhz[k];
+      for (int k = 0; k < KP; ++k) pz[k] = __dmul_rn(wz[k], hz[k]);
+      // wh = sum_z w[z] h[z] in z order (every lane of a group has the same sum)
+      double wh = 0;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const uint32_t z0 = 2 * G * v;
+        if (z0 >= r) break;
+        if (z0 + 2 * G <= r) {
+#pragma unroll
+          for (int l = 0; l < G; ++l) {
+            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
+            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v + 1], l, G));
+          }
+        } else {
+          for (uint32_t l = 0; z0 + 2 * l < r; ++l) {
+            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
+            const double odd = __shfl_sync(kFullMask, pz[2 * v + 1], l, G);
+            if (z0 + 2 * l + 1 < r) wh = __dadd_rn(wh, odd);
+          }
+        }
+      }
+      if (go) {
+        const double f1 = __dmul_rn(em2, __dsub_rn(x, wh));
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const uint32_t z = 2 * (gl + G * v);
+          if (z >= r) continue;
+          double nw[2], nh[2];
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const double t = wz[2 * v + b], u = hz[2 * v + b];
+            if (a.update == kUpdNzsl) {
+              nw[b] = __dsub_rn(t, __dmul_rn(f1, u));
+              nh[b] = __dsub_rn(u, __dmul_rn(f1, t));
+            } else if (a.update == kUpdNzslL2) {
+              nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(__dmul_rn(f2, t), f3)));
+              nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(__dmul_rn(f2, u), f4)));
+            } else {
+              nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(f2, t)));
+              nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(f2, u)));
+            }
+            if (a.truncate) {
+              if (nw[b] <= a.tmin) nw[b] = __dadd_rn(a.tmin, eps);
+              else if (nw[b] >= a.tmax) nw[b] = __dsub_rn(a.tmax, eps);
+              if (nh[b] <= a.tmin) nh[b] = __dadd_rn(a.tmin, eps);
+              else if (nh[b] >= a.tmax) nh[b] = __dsub_rn(a.tmax, eps);
+            }
+          }
+          if (z + 1 >= r) {  // the padding of an odd rank stays zero
+            nw[1] = 0;
+            nh[1] = 0;
+          }
+          *reinterpret_cast<double2*>(w + z) = make_double2(nw[0], nw[1]);
+          *reinterpret_cast<double2*>(h + z) = make_double2(nh[0], nh[1]);
+        }
+      }
     }
   }
 }
 
 // RegularizeL2 (mf/sgd/functions/regularize-l2.h:26-45) applied by every task
 // after sub-epoch s: each W block and the sub-epoch's H blocks are scaled.
-__global__ void regularize_exact_kernel(double* W, double* H, uint64_t m, uint64_t n,
-                                        uint32_t rp, uint32_t r, const uint64_t* off2,
-                                        const uint8_t* mask, uint32_t d, uint32_t nb2,
-                                        const EpochParams* params, double lambda, int truncate,
-                                        double tmin, double tmax) {
+// HBM-bound: 16-byte vectors (rows are padded to whole ones), the row of a
+// vector by a 32-bit division where the sides allow it, the column-block
+// offsets staged in shared memory.
+template <typename I>
+__global__ void __launch_bounds__(256)
+    regularize_exact_kernel(double* W, double* H, uint64_t m, uint64_t n, uint32_t rp, uint32_t r,
+                            const uint64_t* off2, const uint8_t* mask, uint32_t d, uint32_t nb2,
+                            const EpochParams* params, double lambda, int truncate, double tmin,
+                            double tmax) {
+  extern __shared__ __align__(16) uint64_t s_off[];  // nb2 offsets
+  for (uint32_t k = threadIdx.x; k < nb2; k += blockDim.x) s_off[k] = off2[k];
+  __syncthreads();
   const double eps = __ddiv_rn(params->eps, (double)d);  // eps/d: rescaleStratumStepsize()
   double factor = __dsub_rn(1.0, __dmul_rn(__dmul_rn(eps, 2.0), lambda));
   if (factor < 0.5) factor = __ddiv_rn(0.25, __dsub_rn(1.0, factor));
-  const uint64_t wtot = m * rp, htot = n * rp;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < wtot + htot; q += stride) {
-    double* p;
-    uint64_t z;
-    if (q < wtot) {
-      p = W + q;
-      z = q % rp;
-    } else {
-      const uint64_t hq = q - wtot, j = hq / rp;
-      // column block of j
-      uint32_t lo = 0, hi = nb2 - 1;
-      while (lo < hi) {
-        uint32_t mid = (lo + hi + 1) >> 1;
-        if (off2[mid] <= j) lo = mid; else hi = mid - 1;
-      }
-      if (!mask[lo]) continue;
-      p = H + hq;
-      z = hq % rp;
-    }
-    if (z >= r) continue;
-    double v = __dmul_rn(*p, factor);
+  auto scaled = [&](double x) {
+    double v = __dmul_rn(x, factor);
     if (truncate) {
       if (v <= tmin) v = __dadd_rn(tmin, eps);
       else if (v >= tmax) v = __dsub_rn(tmax, eps);
     }
+    return v;
+  };
+  const uint32_t vpr = rp / 2;  // vectors per row
+  const uint64_t wtot = m * vpr, tot = wtot + n * vpr;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < tot; q += stride) {
+    const bool in_w = q < wtot;
+    const I k = (I)(in_w ? q : q - wtot);
+    const I row = k / vpr;
+    if (!in_w) {
+      uint32_t lo = 0, hi = nb2 - 1;  // column block of the row
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (s_off[mid] <= row) lo = mid; else hi = mid - 1;
+      }
+      if (!mask[lo]) continue;
+    }
+    double2* p = reinterpret_cast<double2*>(in_w ? W : H) + k;
+    double2 v = *p;
+    v.x = scaled(v.x);
+    if ((uint32_t)(k - row * vpr) * 2 + 1 < r) v.y = scaled(v.y);  // else padding
     *p = v;
   }
 }
@@ -1045,12 +1172,34 @@ cudaError_t launch_hogwild(int precision, uint32_t lanes, uint32_t vecs, const H
   return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
-cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
-  if (a.r > 32u * kReplayMaxK) return cudaErrorInvalidValue;
-  const uint32_t warps_per_cta = 4;
-  replay_subepoch_kernel<<<(a.d + warps_per_cta - 1) / warps_per_cta, 32 * warps_per_cta, 0, st>>>(
-      a, s);
+namespace {
+
+template <int G, int KP>
+cudaError_t replay_launch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(replay_subepoch_kernel<G, KP>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)replay_smem<G>());
+  if (e != cudaSuccess) return e;
+  replay_subepoch_kernel<G, KP><<<a.d, kReplayThreads, replay_smem<G>(), st>>>(a, s);
   return cudaGetLastError();
+}
+
+}  // namespace
+
+// Lanes per record by rank, for rows of 4 elements per lane up to rank 32 and
+// of 8 above.  Fewer lanes put more records in hand, which helps blocks
+// without repeated rows and columns a little and costs where a hot column
+// lets one record run per round (the posts of those that wait queue): rank
+// 10, 1M uniform entries, d = 4 / 500k Zipf(1.1) entries, d = 16, ms per
+// epoch at 8, 4, 2 lanes: 6.3 / 30, 4.4 / 34, 4.1 / 46; rank 32 and 30 at 8
+// and 4 lanes: 4.1 / 43, 3.7 / 60.
+cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
+  if (a.r <= 16) return replay_launch<4, 4>(a, s, st);
+  if (a.r <= 32) return replay_launch<8, 4>(a, s, st);
+  if (a.r <= 64) return replay_launch<8, 8>(a, s, st);
+  if (a.r <= 128) return replay_launch<16, 8>(a, s, st);
+  if (a.r <= 256) return replay_launch<32, 8>(a, s, st);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_regularize_exact(double* W, double* H, uint64_t m, uint64_t n, uint32_t rp,
@@ -1058,8 +1207,13 @@ cudaError_t launch_regularize_exact(double* W, double* H, uint64_t m, uint64_t n
                                     uint32_t d, uint32_t nb2, const EpochParams* params,
                                     double lambda, int truncate, double tmin, double tmax,
                                     cudaStream_t st) {
-  regularize_exact_kernel<<<1184, 256, 0, st>>>(W, H, m, n, rp, r, off2, mask, d, nb2, params,
-                                                lambda, truncate, tmin, tmax);
+  const size_t smem = sizeof(uint64_t) * nb2;
+  if (std::max(m, n) * (rp / 2) <= 0xffffffffull)
+    regularize_exact_kernel<uint32_t><<<1184, 256, smem, st>>>(
+        W, H, m, n, rp, r, off2, mask, d, nb2, params, lambda, truncate, tmin, tmax);
+  else
+    regularize_exact_kernel<uint64_t><<<1184, 256, smem, st>>>(
+        W, H, m, n, rp, r, off2, mask, d, nb2, params, lambda, truncate, tmin, tmax);
   return cudaGetLastError();
 }
 

@@ -630,3 +630,48 @@ def test_set_counts_replaces_the_update_weights():
         np.testing.assert_array_equal(m1, n1 * 2)
         with pytest.raises(P.DsgdppError):
             b.set_counts(np.full(p.m, 1 << 33, np.uint64), n2)
+
+
+@pytest.mark.parametrize("r,m,n,nnz,d,kind", [
+    (10, 4000, 3000, 60000, 1, "uniform"),   # one task, more than 2^11 rounds' worth of places
+    (16, 300, 200, 9000, 2, "uniform"),      # rows and columns repeat within what is in hand
+    (17, 90, 2, 150, 1, "uniform"),          # two columns: nearly every record waits for another
+    (5, 64, 4000, 30000, 1, "zipf"),         # hot rows and columns: long chains
+    (65, 500, 400, 5000, 3, "zipf"),
+    (200, 300, 200, 3000, 2, "zipf"),
+    (256, 40, 8, 200, 4, "uniform")])        # blocks of a few entries, the widest rows
+def test_replay_runs_independent_records_together_bit_exact(r, m, n, nnz, d, kind):
+    p = _problem(m=m, n=n, nnz=nnz, ntest=10, r=r, kind=kind)
+    ref, ctx = _pair(p, r, d, regularize="L2", regularize_lambda=0.05)
+    with ctx:
+        R = P.Random32(r)
+        for _ in range(2):
+            sched, seeds = P.draw_schedule(R, d, "COWOR")
+            ctx.epoch_explicit(0.01, sched, seeds)
+            ref.epoch_explicit(0.01, sched, seeds)
+        W, H = ctx.get_factors()
+        Wr, Hr = ref.get_factors()
+        np.testing.assert_array_equal(W, Wr)
+        np.testing.assert_array_equal(H, Hr)
+
+
+def test_replay_of_one_column_outlasts_the_round_numbers():
+    # nearly every record lies in one column, so a round runs one or two of
+    # them and the round numbers (2^11) start over
+    rng = np.random.default_rng(3)
+    rows = np.concatenate([np.arange(6000), rng.permutation(6000)[:50]]).astype(np.uint32)
+    cols = np.concatenate([np.zeros(6000), np.ones(50)]).astype(np.uint32)
+    vals = rng.standard_normal(6050)
+    W0, H0 = rng.uniform(-.5, .5, (6000, 7)), rng.uniform(-.5, .5, (2, 7))
+    ref = O.Problem(6000, 2, 7, 1, rows, cols, vals, rows[:5], cols[:5], vals[:5])
+    ref.configure()
+    ref.set_factors(W0, H0)
+    with P.Context(P.Config(m=6000, n=2, rank=7, d=1, precision="fp64", exec="replay",
+                            launch="stream")) as ctx:
+        ctx.set_matrix(P.TRAIN, rows, cols, vals)
+        ctx.set_factors(W0, H0)
+        sched, seeds = P.draw_schedule(P.Random32(5), 1, "WOR")
+        ctx.epoch_explicit(0.001, sched, seeds)
+        ref.epoch_explicit(0.001, sched, seeds)
+        for a, b in zip(ctx.get_factors(), ref.get_factors()):
+            np.testing.assert_array_equal(a, b)
