@@ -202,10 +202,11 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   c->d_mask = dalloc<uint8_t>((size_t)d2 * d2, "mask");
   // one resident wave of the loss kernel; fixed per context, so every loss
   // of the context is reduced in the same order
-  const int loss_per_sm = nzsl_ctas_per_sm(cfg->precision, c->rp);
+  const int loss_per_sm = loss_ctas_per_sm(cfg->precision, c->rp);
   c->loss_grid = (uint32_t)c->num_sms * (uint32_t)std::max(2, std::min(8, loss_per_sm));
   c->d_partials = dalloc<double>(3 * (size_t)c->loss_grid, "partials");
-  c->d_out = dalloc<double>(4, "loss out");
+  c->d_loss_ticket = dalloc<uint32_t>(1, "loss ticket");
+  check_cuda(cudaMemset(c->d_loss_ticket, 0, 4), "loss ticket");
   c->h_out = halloc<double>(4, "loss out");
   check_cuda(cudaEventCreate(&c->ev_begin), "event");
   check_cuda(cudaEventCreate(&c->ev_end), "event");
@@ -250,7 +251,7 @@ void destroy_impl(dsgdpp_ctx* c) {
   hfree(c->h_error);
   hfree(c->h_positions); dfree(c->d_positions); hfree(c->h_pos_offset); dfree(c->d_pos_offset);
   hfree(c->h_mask); dfree(c->d_mask);
-  dfree(c->d_partials); dfree(c->d_out); hfree(c->h_out);
+  dfree(c->d_partials); dfree(c->d_loss_ticket); hfree(c->h_out);
   for (auto e : c->prof_ev) cudaEventDestroy(e);
   c->prof_ev.clear();
   if (c->ev_begin) cudaEventDestroy(c->ev_begin);
@@ -863,81 +864,54 @@ void epoch_explicit_impl(dsgdpp_ctx* c, double eps, const uint32_t* schedule,
 }
 
 // ---- losses --------------------------------------------------------------------------
-double finish_sum(dsgdpp_ctx* c, uint32_t count) {
-  check_cuda(launch_sum_partials(c->d_partials, count, c->d_out, c->stream), "sum_partials");
-  check_cuda(cudaMemcpyAsync(c->h_out, c->d_out, 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
+// Launches the squared errors of the training or test entries (which < 0: of
+// none) with the terms `reg` (LossArgs) of the factors into out[0 .. 2], a part
+// of the pinned h_out that holds them once the stream is synchronised.
+void enqueue_loss(dsgdpp_ctx* c, int which, int reg, double* out) {
+  LossArgs a{};
+  if (which >= 0) {
+    if (which != DSGDPP_TRAIN && which != DSGDPP_TEST) throw Error(DSGDPP_E_INVALID, "which");
+    const DevMatrix& M = c->mat[which];
+    if (!M.present) throw Error(DSGDPP_E_STATE, which ? "no test matrix" : "no training matrix");
+    a.row = M.row; a.col = M.col; a.val = M.val; a.nnz = M.nnz;
+  }
+  a.W = c->W; a.H = c->H;
+  a.m = c->cfg.m; a.n = c->cfg.n;
+  a.r = c->r; a.rp = c->rp;
+  a.zero_pad = true;
+  a.reg = reg;
+  a.cnt1 = c->cnt1; a.cnt2 = c->cnt2;
+  a.partials = c->d_partials;
+  a.ticket = c->d_loss_ticket;
+  a.out = out;
+  check_cuda(cudaSetDevice(c->cfg.device), "cudaSetDevice");
+  check_cuda(launch_loss(c->cfg.precision, a, c->loss_grid, c->stream), "loss");
+}
+
+double nzsl_impl(dsgdpp_ctx* c, int which) {
+  if (which != DSGDPP_TRAIN && which != DSGDPP_TEST) throw Error(DSGDPP_E_INVALID, "which");
+  enqueue_loss(c, which, 0, c->h_out);
   check_cuda(cudaStreamSynchronize(c->stream), "sync");
   return c->h_out[0];
 }
 
-// Sums n consecutive runs of loss_grid partials into d_out[0..n) and reads
-// them back with one copy and one synchronisation.
-void finish_sums(dsgdpp_ctx* c, uint32_t n, double* out) {
-  for (uint32_t k = 0; k < n; ++k)
-    check_cuda(launch_sum_partials(c->d_partials + (size_t)k * c->loss_grid, c->loss_grid,
-                                   c->d_out + k, c->stream), "sum_partials");
-  check_cuda(cudaMemcpyAsync(c->h_out, c->d_out, 8 * (size_t)n, cudaMemcpyDeviceToHost, c->stream),
-             "D2H");
+// The terms `reg` of W and of H.
+void factor_terms(dsgdpp_ctx* c, int reg, double* w, double* h) {
+  enqueue_loss(c, -1, reg, c->h_out);
   check_cuda(cudaStreamSynchronize(c->stream), "sync");
-  for (uint32_t k = 0; k < n; ++k) out[k] = c->h_out[k];
+  if (w) *w = c->h_out[1];
+  if (h) *h = c->h_out[2];
 }
 
-// The squared errors of the training or test entries as loss_grid partials.
-void nzsl_partials(dsgdpp_ctx* c, int which, double* partials) {
-  if (which != DSGDPP_TRAIN && which != DSGDPP_TEST) throw Error(DSGDPP_E_INVALID, "which");
-  const DevMatrix& M = c->mat[which];
-  if (!M.present) throw Error(DSGDPP_E_STATE, which ? "no test matrix" : "no training matrix");
-  check_cuda(cudaSetDevice(c->cfg.device), "cudaSetDevice");
-  if (M.nnz == 0) {
-    check_cuda(cudaMemsetAsync(partials, 0, sizeof(double) * c->loss_grid, c->stream), "memset");
-    return;
-  }
-  check_cuda(launch_nzsl_partials(c->cfg.precision, M.row, M.col, M.val, M.nnz, c->W, c->H, c->r,
-                                  c->rp, partials, c->loss_grid, c->stream), "nzsl");
-}
-
-double nzsl_impl(dsgdpp_ctx* c, int which) {
-  nzsl_partials(c, which, c->d_partials);
-  double v = 0;
-  finish_sums(c, 1, &v);
-  return v;
-}
-
-double sumsq_impl(dsgdpp_ctx* c, const void* X, uint64_t count) {
-  check_cuda(launch_sumsq_partials(c->cfg.precision, X, count, c->d_partials, c->loss_grid,
-                                   c->stream), "l2");
-  return finish_sum(c, c->loss_grid);
-}
-
-double nzl2_impl(dsgdpp_ctx* c, const void* X, uint64_t rows, const uint32_t* cnt) {
-  check_cuda(launch_nzl2_partials(c->cfg.precision, X, rows, c->rp, cnt, c->d_partials,
-                                  c->loss_grid, c->stream), "nzl2");
-  return finish_sum(c, c->loss_grid);
-}
-
-// The configured loss (mf/loss/loss.h:88-112 SumLoss of Nzsl and L2/Nzl2):
-// its two or three reductions run back to back and come back in one copy.
+// The configured loss (mf/loss/loss.h:88-112 SumLoss of Nzsl and L2/Nzl2).
 double loss_impl(dsgdpp_ctx* c) {
-  const uint32_t G = c->loss_grid;
-  nzsl_partials(c, DSGDPP_TRAIN, c->d_partials);
-  uint32_t n = 1;
-  if (c->cfg.loss == DSGDPP_LOSS_NZSL_L2) {
-    check_cuda(launch_sumsq_partials(c->cfg.precision, c->W, c->cfg.m * c->rp, c->d_partials + G,
-                                     G, c->stream), "l2");
-    check_cuda(launch_sumsq_partials(c->cfg.precision, c->H, c->cfg.n * c->rp,
-                                     c->d_partials + 2 * (size_t)G, G, c->stream), "l2");
-    n = 3;
-  } else if (c->cfg.loss == DSGDPP_LOSS_NZSL_NZL2) {
-    check_cuda(launch_nzl2_partials(c->cfg.precision, c->W, c->cfg.m, c->rp, c->cnt1,
-                                    c->d_partials + G, G, c->stream), "nzl2");
-    check_cuda(launch_nzl2_partials(c->cfg.precision, c->H, c->cfg.n, c->rp, c->cnt2,
-                                    c->d_partials + 2 * (size_t)G, G, c->stream), "nzl2");
-    n = 3;
-  }
-  double v[3] = {0, 0, 0};
-  finish_sums(c, n, v);
-  double l = v[0];
-  if (n == 3) l = l + c->cfg.loss_lambda * (v[1] + v[2]);
+  const int reg = c->cfg.loss == DSGDPP_LOSS_NZSL_L2     ? 1
+                  : c->cfg.loss == DSGDPP_LOSS_NZSL_NZL2 ? 2
+                                                         : 0;
+  enqueue_loss(c, DSGDPP_TRAIN, reg, c->h_out);
+  check_cuda(cudaStreamSynchronize(c->stream), "sync");
+  double l = c->h_out[0];
+  if (reg) l = l + c->cfg.loss_lambda * (c->h_out[1] + c->h_out[2]);
   return l;
 }
 
@@ -1365,8 +1339,7 @@ int dsgdpp_l2(dsgdpp_ctx* c, double* w2, double* h2) {
   TraceRange range("loss");
   return guarded(c, [&]() {
     check_cuda(cudaSetDevice(c->cfg.device), "cudaSetDevice");
-    if (w2) *w2 = sumsq_impl(c, c->W, c->cfg.m * c->rp);
-    if (h2) *h2 = sumsq_impl(c, c->H, c->cfg.n * c->rp);
+    factor_terms(c, 1, w2, h2);
     return DSGDPP_OK;
   });
 }
@@ -1376,8 +1349,7 @@ int dsgdpp_nzl2(dsgdpp_ctx* c, double* w, double* h) {
   return guarded(c, [&]() {
     if (!c->mat[0].present) throw Error(DSGDPP_E_STATE, "no training matrix");
     check_cuda(cudaSetDevice(c->cfg.device), "cudaSetDevice");
-    if (w) *w = nzl2_impl(c, c->W, c->cfg.m, c->cnt1);
-    if (h) *h = nzl2_impl(c, c->H, c->cfg.n, c->cnt2);
+    factor_terms(c, 2, w, h);
     return DSGDPP_OK;
   });
 }
@@ -1463,19 +1435,12 @@ int dsgdpp_update_norms(dsgdpp_ctx* c, double* mean, double* max) {
   return guarded(c, [&]() {
     if (!c->W_saved) throw Error(DSGDPP_E_STATE, "no saved factors");
     check_cuda(cudaSetDevice(c->cfg.device), "cudaSetDevice");
-    double sum = 0, mx = 0;
-    const struct { const void* x; const void* old; uint64_t rows; } parts[2] = {
-        {c->W, c->W_saved, c->cfg.m}, {c->H, c->H_saved, c->cfg.n}};
-    for (const auto& p : parts) {
-      check_cuda(launch_update_norms(c->cfg.precision, p.x, p.old, p.rows, c->rp, c->d_partials,
-                                     c->loss_grid, c->d_out, c->stream), "update norms");
-      check_cuda(cudaMemcpyAsync(c->h_out, c->d_out, 16, cudaMemcpyDeviceToHost, c->stream), "D2H");
-      check_cuda(cudaStreamSynchronize(c->stream), "sync");
-      sum += c->h_out[0];
-      mx = std::max(mx, c->h_out[1]);
-    }
-    if (mean) *mean = sum / (double)(c->cfg.m + c->cfg.n);
-    if (max) *max = mx;
+    check_cuda(launch_update_norms(c->cfg.precision, c->W, c->W_saved, c->cfg.m, c->H, c->H_saved,
+                                   c->cfg.n, c->rp, c->d_partials, c->loss_grid, c->d_loss_ticket,
+                                   c->h_out, c->stream), "update norms");
+    check_cuda(cudaStreamSynchronize(c->stream), "sync");
+    if (mean) *mean = c->h_out[0] / (double)(c->cfg.m + c->cfg.n);
+    if (max) *max = c->h_out[1];
     return DSGDPP_OK;
   });
 }

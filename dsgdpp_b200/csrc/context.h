@@ -123,8 +123,8 @@ struct dsgdpp_ctx {
   uint8_t* d_mask = nullptr;
   // losses
   double* d_partials = nullptr;
-  double* d_out = nullptr;
-  double* h_out = nullptr;
+  uint32_t* d_loss_ticket = nullptr;
+  double* h_out = nullptr;  // pinned: the loss kernels write their results here
   uint32_t loss_grid = 0;
   // Hogwild launch shape
   uint32_t lanes = 0, vecs = 0, grid = 0;

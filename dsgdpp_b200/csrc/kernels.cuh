@@ -141,19 +141,33 @@ cudaError_t launch_scale_rows(int precision, void* W, uint64_t wrows, void* H, u
                               uint32_t rp, const uint32_t* w_slot, const uint32_t* h_slot,
                               const float* scales, cudaStream_t st);
 
-// Loss partial sums (FP64); `partials` holds `grid` doubles, then sum_partials
-// writes the total to out[0].
-cudaError_t launch_nzsl_partials(int precision, const uint32_t* row, const uint32_t* col,
-                                 const void* val, uint64_t nnz, const void* W, const void* H,
-                                 uint32_t r, uint32_t rp, double* partials, uint32_t grid,
-                                 cudaStream_t st);
-// CTAs per SM of the training-loss kernel for this precision and row width
-int nzsl_ctas_per_sm(int precision, uint32_t rp);
-cudaError_t launch_sumsq_partials(int precision, const void* X, uint64_t count,
-                                  double* partials, uint32_t grid, cudaStream_t st);
-cudaError_t launch_nzl2_partials(int precision, const void* X, uint64_t rows, uint32_t rp,
-                                 const uint32_t* cnt, double* partials, uint32_t grid,
-                                 cudaStream_t st);
+// A loss in one launch: the squared errors of the entries, and with `reg` the
+// sums of squares of W and H (1) or their count-weighted forms (2).  With a
+// ticket (a zeroed word that the launch leaves zeroed) out[0 .. 2] (out[0]
+// without `reg`; device or pinned host memory) get the sums, and `partials`
+// holds 3 * grid doubles; without one the squared errors stay in partials[0 ..
+// grid) for sum_partials.
+struct LossArgs {
+  const uint32_t* row;
+  const uint32_t* col;
+  const void* val;  // float (FP32 / BF16 factors) or double
+  uint64_t nnz;
+  const void* W;
+  const void* H;
+  uint64_t m, n;
+  uint32_t r, rp;
+  bool zero_pad;         // rows hold zeros from r to rp (FP32 / BF16)
+  int reg;
+  const uint32_t* cnt1;  // reg 2: nnz1, nnz2
+  const uint32_t* cnt2;
+  double* partials;
+  uint32_t* ticket;
+  double* out;
+};
+cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st);
+// CTAs per SM of the loss kernel for this precision and row width
+int loss_ctas_per_sm(int precision, uint32_t rp);
+// out[0] = the sum of `count` partials
 cudaError_t launch_sum_partials(const double* partials, uint32_t count, double* out,
                                 cudaStream_t st);
 
@@ -172,10 +186,12 @@ cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_
 cudaError_t launch_owner_sums(const double* partials, const uint32_t* owner_begin,
                               uint32_t owners, double* out, cudaStream_t st);
 
-// Sum (out2[0]) and maximum (out2[1]) over rows of |X_i - Xold_i|; partials
-// holds 2 * grid doubles.
-cudaError_t launch_update_norms(int precision, const void* X, const void* Xold, uint64_t rows,
-                                uint32_t rp, double* partials, uint32_t grid, double* out2,
+// Sum (out[0]) and maximum (out[1]) over the rows of W and of H of their
+// Euclidean move since W0, H0; partials holds 2 * grid doubles, ticket and out
+// as in LossArgs.
+cudaError_t launch_update_norms(int precision, const void* W, const void* W0, uint64_t m,
+                                const void* H, const void* H0, uint64_t n, uint32_t rp,
+                                double* partials, uint32_t grid, uint32_t* ticket, double* out,
                                 cudaStream_t st);
 
 // ---- step-size controller network (16 -> 64 -> 64 -> 1, GELU) -----------------------

@@ -13,10 +13,6 @@
 namespace dsgdpp {
 namespace {
 
-inline uint32_t vec_width_of(int precision) {
-  return precision == kFp64 ? 2 : (precision == kFp32 ? 4 : 8);
-}
-
 __device__ __forceinline__ double block_reduce(double v, double* sh) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFullMask, v, off);
@@ -32,79 +28,199 @@ __device__ __forceinline__ double block_reduce(double v, double* sh) {
   return t;  // valid in thread 0
 }
 
-template <typename T, typename V>
-__global__ void __launch_bounds__(256) nzsl_partials_kernel(const uint32_t* row, const uint32_t* col,
-                                                            const V* val, uint64_t nnz, const T* W,
-                                                            const T* H, uint32_t r, uint32_t rp,
-                                                            double* partials) {
-  using E = Elem<T>;
-  constexpr int VW = E::VW;
-  __shared__ double sh[32];
-  double acc = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < nnz; k += stride) {
-    const T* w = W + (size_t)row[k] * rp;
-    const T* h = H + (size_t)col[k] * rp;
-    double ip = 0;
-    for (uint32_t z0 = 0; z0 < r; z0 += VW) {
-      typename E::C wf[VW], hf[VW];
-      E::unpack(*reinterpret_cast<const uint4*>(w + z0), wf);
-      E::unpack(*reinterpret_cast<const uint4*>(h + z0), hf);
+__device__ __forceinline__ double block_max(double v, double* sh) {
 #pragma unroll
-      for (int e = 0; e < VW; ++e)
-        if (z0 + e < r) ip = __dadd_rn(ip, __dmul_rn((double)wf[e], (double)hf[e]));
-    }
-    const double diff = __dsub_rn((double)val[k], ip);
-    acc = __dadd_rn(acc, __dmul_rn(diff, diff));
+  for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(kFullMask, v, off));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) sh[warp] = v;
+  __syncthreads();
+  double t = 0;
+  if (warp == 0) {
+    t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t = fmax(t, __shfl_xor_sync(kFullMask, t, off));
   }
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+  return t;  // valid in thread 0
 }
 
-// FP32 / BF16 factors: LPN lanes per entry, each lane loading VPL 16-byte
-// vectors of the W row and H column, so a row is one coalesced request.  A
-// warp takes 32 consecutive entries (one index load per lane), then walks
-// them in LPN rounds of 32 / LPN entries, the factor loads of U rounds issued
-// before any is used.  Products of two floats are exact in FP64; each lane
-// sums its elements in z order and the group adds the lane sums by a fixed
-// butterfly.  Entries [begin, end) are dealt to warps warp, warp + nwarps, ...
-// 32 at a time; a warp loads its next 32 entries before it sums the current
-// ones.  Training loss on 100M entries at rank 32: 2.97 -> 2.30 ms (FP32) and
-// 2.21 -> 2.10 ms (BF16) with the entries in flight, then 2.15 and 1.83 ms
-// with H built by f32_scaled (99M entries at rank 128: 8.17 -> 6.97 ms FP32,
-// 6.81 -> 5.05 ms BF16).
 // f * 2^-896 as a double, exactly, built from the float's bits with integer
 // operations: the 8-bit exponent field and 23-bit fraction move into the low
 // bits of the double's exponent field and the top of its fraction, so an
 // exponent field e reads as 2^(e-1023) where the float meant 2^(e-127) --
-// for normal and subnormal floats alike.  The conversion unit, which bounds
-// the loss kernels (two conversions per product), then converts only W.
-__device__ __forceinline__ double f32_scaled(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const uint32_t hi = ((b >> 3) & 0x0fffffffu) | (b & 0x80000000u);
-  return __hiloint2double((int)hi, (int)(b << 29));
+// for normal and subnormal floats alike.  The conversion unit (16 values per
+// clock and SM), which bounds the loss kernels, then converts only W.  (The
+// arithmetic shift brings the sign along; the mask clears its copies.)
+__device__ __forceinline__ double f32_scaled(uint32_t b) {
+  return __hiloint2double(((int)b >> 3) & (int)0x8fffffffu, (int)(b << 29));
 }
 
-template <typename T, int LPN, int VPL>
-__device__ __forceinline__ double nzsl_lanes(const uint32_t* row, const uint32_t* col,
-                                             const float* val, const T* W, const T* H,
-                                             uint32_t r, uint32_t rp, uint64_t begin,
+// ---- squared errors, FP32 / BF16 factors ------------------------------------------
+// A warp takes 32 consecutive entries (one index load per lane, the next 32
+// loaded while these are summed) and walks them in L rounds of 32 / L, L lanes
+// per entry with V vectors of the W row and of the H column each.  Products of
+// two floats are exact in FP64; each lane sums its elements in z order.  The
+// lane sums of the L rounds are then added by a transposing butterfly -- each
+// step halves the values a lane holds -- that leaves every lane with the inner
+// product of one entry, so the difference and its square are formed once per
+// 32 entries on all lanes.
+//
+// L is chosen so that one load instruction covers 128 contiguous bytes of a
+// row (4 lanes of 32 bytes where rows are whole 32-byte vectors): an L1 lookup
+// handles one line at a time, and 16 rows of 32 bytes per instruction cost
+// four times the lookups.
+//
+// Bound: no single unit -- on 20M Zipf(1.1) entries at rank 32 the L1 data
+// path is 68% busy, instruction issue 53%, the conversion unit and the integer
+// pipe 49%.  Measured there against 2 lanes with four 16-byte vectors, a full
+// butterfly per round and zero-filled, predicated loads (ms per loss without
+// factor terms): FP32 rank 10 0.40 -> 0.22, 16 0.33 -> 0.20, 32 0.45 -> 0.31,
+// 50 0.75 -> 0.61, 64 0.73 -> 0.55, 128 1.47 -> 1.05; BF16 rank 32 0.39 ->
+// 0.27, 64 0.57 -> 0.48, 128 1.05 -> 0.83.  100M entries at rank 32: 2.21 ->
+// 1.54 ms.
+template <int N>
+struct Words {
+  uint32_t w[N];
+};
+template <int N>
+__device__ __forceinline__ Words<N> load_words(const void* p) {
+  Words<N> r;
+  if constexpr (N == 8) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]),
+          "=r"(r.w[6]), "=r"(r.w[7])
+        : "l"(p));
+  } else {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w;
+  }
+  return r;
+}
+// element e of a vector, as the bits of a float
+template <typename T, int N>
+__device__ __forceinline__ uint32_t elem_bits(const Words<N>& v, int e) {
+  if constexpr (sizeof(T) == 4) return v.w[e];
+  else return (e & 1) ? v.w[e / 2] & 0xffff0000u : v.w[e / 2] << 16;
+}
+
+// vector words of each side that a lane has in flight (8: 0.27 against 0.26 ms
+// at BF16 rank 32; 32 spill, or halve the warps)
+constexpr int kLossWords = 16;
+
+struct Entries {
+  const uint32_t* row;
+  const uint32_t* col;
+  const float* val;
+};
+
+// The squared error of 32 entries (nrec of them exist), one entry per lane in
+// the end.  FAST: all 32 exist and rows are padded with zeros, so whole vectors
+// are summed; a lane past the row's end reads its first vector and drops it.
+template <typename T, int L, int V, int N, bool FAST>
+__device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, float my_val,
+                                            uint32_t nrec, const T* W, const T* H, uint32_t r,
+                                            uint32_t rp) {
+  constexpr int NG = 32 / L;                       // entries per round
+  constexpr int EPV = N * 4 / (int)sizeof(T);      // elements per vector
+  // vectors of each side that a lane has in flight: U rounds of a row's V, or
+  // C of one round's
+  constexpr int F = kLossWords / N;
+  constexpr int C = V < F ? V : F;
+  constexpr int U = F / V < 1 ? 1 : F / V < L ? F / V : L;
+  const uint32_t lane = threadIdx.x & 31u, grp = lane / L, gl = lane % L;
+  double ip[L];
+#pragma unroll
+  for (int t0 = 0; t0 < L; t0 += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) ip[t0 + u] = 0;
+#pragma unroll
+    for (int v0 = 0; v0 < V; v0 += C) {
+      Words<N> wv[U][C], hv[U][C];
+      if (t0 + v0) asm volatile("" ::: "memory");  // no more loads ahead than planned
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t ri = (t0 + u) * NG + grp;
+        const T* w = W + (size_t)__shfl_sync(kFullMask, my_row, ri) * rp;
+        const T* h = H + (size_t)__shfl_sync(kFullMask, my_col, ri) * rp;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          if (v0 + c >= V) continue;
+          const uint32_t z0 = (uint32_t)((v0 + c) * L + gl) * EPV;
+          if constexpr (FAST) {
+            const uint32_t at = v0 + c < V - 1 || z0 < rp ? z0 : 0;  // only the last may not exist
+            wv[u][c] = load_words<N>(w + at);
+            hv[u][c] = load_words<N>(h + at);
+          } else {
+            wv[u][c] = Words<N>{};
+            hv[u][c] = Words<N>{};
+            if (ri < nrec && z0 < rp) {
+              wv[u][c] = load_words<N>(w + z0);
+              hv[u][c] = load_words<N>(h + z0);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        double s = ip[t0 + u];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          if (v0 + c >= V) continue;
+          const uint32_t z0 = (uint32_t)((v0 + c) * L + gl) * EPV;
+          // The product of two floats is exact in FP64, so the fused
+          // multiply-add rounds exactly like the separate add.  The sum is
+          // formed with H scaled by 2^-896 and scaled back once: a power of
+          // two, so it rounds exactly as unscaled wherever the scaled terms
+          // stay normal doubles (magnitudes of 2^-126 and up; below that the
+          // absolute error stays under 2^-178).
+          if (FAST || z0 + EPV <= r) {
+            const double before = s;
+#pragma unroll
+            for (int e = 0; e < EPV; ++e)
+              s = fma((double)__uint_as_float(elem_bits<T>(wv[u][c], e)),
+                      f32_scaled(elem_bits<T>(hv[u][c], e)), s);
+            if (FAST && v0 + c == V - 1 && z0 >= rp) s = before;
+          } else {
+#pragma unroll
+            for (int e = 0; e < EPV; ++e)
+              if (z0 + e < r)
+                s = fma((double)__uint_as_float(elem_bits<T>(wv[u][c], e)),
+                        f32_scaled(elem_bits<T>(hv[u][c], e)), s);
+          }
+        }
+        ip[t0 + u] = s;
+      }
+    }
+  }
+#pragma unroll
+  for (int off = L / 2; off > 0; off >>= 1) {
+    const bool up = (gl & off) != 0;
+#pragma unroll
+    for (int k = 0; k < off; ++k) {
+      const double keep = up ? ip[k + off] : ip[k], send = up ? ip[k] : ip[k + off];
+      ip[k] = __dadd_rn(keep, __shfl_xor_sync(kFullMask, send, off));
+    }
+  }
+  // this lane's entry: round gl of its group
+  const uint32_t ri = gl * NG + grp;
+  const float x = __shfl_sync(kFullMask, my_val, ri);
+  const double diff = __dsub_rn((double)x, __dmul_rn(ip[0], 0x1p896));
+  return FAST || ri < nrec ? __dmul_rn(diff, diff) : 0.0;
+}
+
+// Entries [begin, end) dealt to warps warp, warp + nwarps, ... 32 at a time.
+template <typename T, int L, int V, int N>
+__device__ __forceinline__ double nzsl_lanes(const Entries& en, const T* W, const T* H, uint32_t r,
+                                             uint32_t rp, bool zero_pad, uint64_t begin,
                                              uint64_t end, uint64_t warp, uint64_t nwarps) {
-  using E = Elem<T>;
-  constexpr int VW = E::VW;
-  constexpr int NG = 32 / LPN;          // entries per round
-  // rounds with loads in flight together (bounded by the registers they hold)
-  constexpr int U = VPL == 1 ? (LPN < 4 ? LPN : 4) : (VPL == 2 ? 2 : 1);
-  const uint32_t lane = threadIdx.x & 31u, grp = lane / LPN, gl = lane % LPN;
-  const uint32_t nvec = rp / VW;
+  const uint32_t lane = threadIdx.x & 31u;
   double acc = 0;
   uint64_t base = begin + warp * 32;
   uint32_t n_row = 0, n_col = 0;
   float n_val = 0;
   if (base + lane < end) {
-    n_row = row[base + lane];
-    n_col = col[base + lane];
-    n_val = val[base + lane];
+    n_row = en.row[base + lane];
+    n_col = en.col[base + lane];
+    n_val = en.val[base + lane];
   }
   for (; base < end; base += nwarps * 32) {
     const uint32_t my_row = n_row, my_col = n_col;
@@ -112,86 +228,21 @@ __device__ __forceinline__ double nzsl_lanes(const uint32_t* row, const uint32_t
     // the next 32 entries travel while these are summed
     const uint64_t nk = base + nwarps * 32 + lane;
     if (nk < end) {
-      n_row = row[nk];
-      n_col = col[nk];
-      n_val = val[nk];
+      n_row = en.row[nk];
+      n_col = en.col[nk];
+      n_val = en.val[nk];
     }
     const uint32_t nrec = (uint32_t)min((uint64_t)32, end - base);
-#pragma unroll 1
-    for (uint32_t t0 = 0; t0 < (uint32_t)LPN; t0 += U) {
-      uint4 wv[U][VPL], hv[U][VPL];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t ri = (t0 + u) * NG + grp;
-        const uint32_t rr = __shfl_sync(kFullMask, my_row, ri);
-        const uint32_t cc = __shfl_sync(kFullMask, my_col, ri);
-        const bool valid = ri < nrec;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const uint32_t vi = v * LPN + gl;
-          if (valid && vi < nvec) {
-            wv[u][v] = __ldg(reinterpret_cast<const uint4*>(W + (size_t)rr * rp + vi * VW));
-            hv[u][v] = __ldg(reinterpret_cast<const uint4*>(H + (size_t)cc * rp + vi * VW));
-          } else {
-            wv[u][v] = make_uint4(0, 0, 0, 0);
-            hv[u][v] = make_uint4(0, 0, 0, 0);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t ri = (t0 + u) * NG + grp;
-        double ip = 0;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          float wf[VW], hf[VW];
-          E::unpack(wv[u][v], wf);
-          E::unpack(hv[u][v], hf);
-          const uint32_t z0 = (v * LPN + gl) * VW;
-          // The product of two floats is exact in FP64, so the fused
-          // multiply-add rounds exactly like the separate add.  The sum is
-          // formed with H scaled by 2^-896 and scaled back once: a power of
-          // two, so it rounds exactly as unscaled wherever the scaled terms
-          // stay normal doubles (magnitudes of 2^-126 and up; below that the
-          // absolute error stays under 2^-178).
-          if (z0 + VW <= r) {
-#pragma unroll
-            for (int e = 0; e < VW; ++e) ip = fma((double)wf[e], f32_scaled(hf[e]), ip);
-          } else {
-#pragma unroll
-            for (int e = 0; e < VW; ++e)
-              if (z0 + e < r) ip = fma((double)wf[e], f32_scaled(hf[e]), ip);
-          }
-        }
-        ip = __dmul_rn(ip, 0x1p896);
-#pragma unroll
-        for (int off = LPN / 2; off > 0; off >>= 1)
-          ip = __dadd_rn(ip, __shfl_xor_sync(kFullMask, ip, off));
-        const float x = __shfl_sync(kFullMask, my_val, ri);
-        if (ri < nrec && gl == 0) {
-          const double diff = __dsub_rn((double)x, ip);
-          acc = __dadd_rn(acc, __dmul_rn(diff, diff));
-        }
-      }
-    }
+    acc = __dadd_rn(acc, nrec == 32 && zero_pad
+                             ? squares32<T, L, V, N, true>(my_row, my_col, my_val, nrec, W, H, r, rp)
+                             : squares32<T, L, V, N, false>(my_row, my_col, my_val, nrec, W, H, r,
+                                                            rp));
   }
   return acc;
 }
 
-template <typename T, int LPN, int VPL>
-__global__ void __launch_bounds__(256, 3)
-    nzsl_lanes_kernel(const uint32_t* row, const uint32_t* col, const float* val, uint64_t nnz,
-                      const T* W, const T* H, uint32_t r, uint32_t rp, double* partials) {
-  __shared__ double sh[32];
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const double acc = nzsl_lanes<T, LPN, VPL>(row, col, val, W, H, r, rp, 0, nnz, warp, warps);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-
 // FP64 factors: one thread per entry, the inner product in z order (as the
-// reference forms it) over entries [begin, end) dealt by `stride`.
+// reference forms it, no contraction) over entries first, first + stride, ...
 __device__ __forceinline__ double nzsl_exact(const uint32_t* row, const uint32_t* col,
                                              const double* val, const double* W, const double* H,
                                              uint32_t r, uint32_t rp, uint64_t first,
@@ -201,109 +252,16 @@ __device__ __forceinline__ double nzsl_exact(const uint32_t* row, const uint32_t
     const double* w = W + (size_t)row[k] * rp;
     const double* h = H + (size_t)col[k] * rp;
     double ip = 0;
-    for (uint32_t z = 0; z < r; ++z) ip = __dadd_rn(ip, __dmul_rn(w[z], h[z]));
+    for (uint32_t z = 0; z < r; z += 2) {
+      const double2 a = *reinterpret_cast<const double2*>(w + z);
+      const double2 b = *reinterpret_cast<const double2*>(h + z);
+      ip = __dadd_rn(ip, __dmul_rn(a.x, b.x));
+      if (z + 1 < r) ip = __dadd_rn(ip, __dmul_rn(a.y, b.y));
+    }
     const double diff = __dsub_rn(val[k], ip);
     acc = __dadd_rn(acc, __dmul_rn(diff, diff));
   }
   return acc;
-}
-
-// ---- per-problem (segmented) reductions of the batched form ----------------------
-// One CTA per chunk of a problem's range; owner_sums then adds each problem's
-// chunk partials in chunk order, so every per-problem sum is deterministic.
-template <typename T, int LPN, int VPL>
-__global__ void __launch_bounds__(256, 3) nzsl_chunks_kernel(const RangeChunk* chunks,
-                                                          const uint32_t* row, const uint32_t* col,
-                                                          const float* val, const T* W,
-                                                          const T* H, uint32_t r, uint32_t rp,
-                                                          double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  const double acc = nzsl_lanes<T, LPN, VPL>(row, col, val, W, H, r, rp, c.begin, c.end,
-                                             threadIdx.x >> 5, blockDim.x >> 5);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-__global__ void __launch_bounds__(256) nzsl_chunks_exact_kernel(
-    const RangeChunk* chunks, const uint32_t* row, const uint32_t* col, const double* val,
-    const double* W, const double* H, uint32_t r, uint32_t rp, double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  const double acc =
-      nzsl_exact(row, col, val, W, H, r, rp, c.begin + threadIdx.x, c.end, blockDim.x);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-template <typename T>
-__global__ void __launch_bounds__(256) sumsq_chunks_kernel(const RangeChunk* chunks, const T* X,
-                                                           double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  double acc = 0;
-  for (uint64_t k = c.begin + threadIdx.x; k < c.end; k += blockDim.x) {
-    const double v = (double)(float)X[k];
-    acc = __dadd_rn(acc, __dmul_rn(v, v));
-  }
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-template <>
-__global__ void __launch_bounds__(256) sumsq_chunks_kernel<double>(const RangeChunk* chunks,
-                                                                   const double* X,
-                                                                   double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  double acc = 0;
-  for (uint64_t k = c.begin + threadIdx.x; k < c.end; k += blockDim.x)
-    acc = __dadd_rn(acc, __dmul_rn(X[k], X[k]));
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-__global__ void __launch_bounds__(256) owner_sums_kernel(const double* partials,
-                                                         const uint32_t* owner_begin,
-                                                         double* out) {
-  __shared__ double sh[32];
-  const uint32_t p = blockIdx.x;
-  double acc = 0;
-  for (uint32_t k = owner_begin[p] + threadIdx.x; k < owner_begin[p + 1]; k += blockDim.x)
-    acc = __dadd_rn(acc, partials[k]);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) out[p] = t;
-}
-
-// lane mapping of the FP32 / BF16 loss kernels: LPN = the power of two
-// covering the row's vectors (at most 32), VPL = vectors per lane
-struct LossShape {
-  uint32_t lanes, vecs;
-};
-LossShape loss_shape(uint32_t nvec) {
-  // rows of up to 4 vectors: one vector per lane; longer rows: 4 vectors per
-  // lane, so fewer lanes share an entry and the butterfly is shorter (measured
-  // faster at rank 32 FP32 and rank 128, slower at rank 32 BF16)
-  LossShape s{2, 1};
-  s.vecs = nvec > 4 ? 4 : 1;
-  while (s.lanes * s.vecs < nvec && s.lanes < 32) s.lanes <<= 1;
-  s.vecs = (nvec + s.lanes - 1) / s.lanes;
-  if (s.vecs == 3) s.vecs = 4;
-  return s;
-}
-
-template <typename T>
-void* nzsl_lanes_fn(LossShape s, bool chunks) {
-#define DSGDPP_CASE(L, V)                                                            \
-  if (s.lanes == L && s.vecs == V)                                                   \
-    return chunks ? reinterpret_cast<void*>(&nzsl_chunks_kernel<T, L, V>)            \
-                  : reinterpret_cast<void*>(&nzsl_lanes_kernel<T, L, V>);
-  DSGDPP_CASE(2, 1) DSGDPP_CASE(4, 1) DSGDPP_CASE(2, 4) DSGDPP_CASE(4, 4)
-  DSGDPP_CASE(8, 4) DSGDPP_CASE(16, 4) DSGDPP_CASE(32, 4)
-#undef DSGDPP_CASE
-  return nullptr;
-}
-
-void* nzsl_fn(int precision, uint32_t rp, bool chunks) {
-  const LossShape s = loss_shape(rp / vec_width_of(precision));
-  return precision == kFp32 ? nzsl_lanes_fn<float>(s, chunks)
-                            : nzsl_lanes_fn<__nv_bfloat16>(s, chunks);
 }
 
 // Squares of the elements of one 16-byte vector, added in element order.
@@ -325,19 +283,16 @@ __device__ __forceinline__ double add_squares(double acc, const uint4& v) {
   return acc;
 }
 
-// Sum of squares of `count` factor entries (L2Loss, mf/loss/l2.h) in FP64:
-// 16-byte vector loads dealt grid-stride to the threads, four vectors in
-// flight per thread; the elements past the last whole vector (none when rows
-// are padded to a vector) go to the first threads.
+// Sum of squares of `count` factor elements (L2Loss, mf/loss/l2.h) dealt to
+// threads tid, tid + stride, ...: 16-byte loads, four in flight per thread; the
+// elements past the last whole vector (none when rows are padded to a vector)
+// go to the first threads.
 template <typename T>
-__global__ void __launch_bounds__(256) sumsq_partials_kernel(const T* X, uint64_t count,
-                                                             double* partials) {
-  __shared__ double sh[32];
+__device__ __forceinline__ double sum_squares(const T* X, uint64_t count, uint64_t tid,
+                                              uint64_t stride) {
   constexpr int VW = Elem<T>::VW;
   const uint4* V = reinterpret_cast<const uint4*>(X);
   const uint64_t nvec = count / VW;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   double acc = 0;
   uint64_t k = tid;
   for (; k + 3 * stride < nvec; k += 4 * stride) {
@@ -352,32 +307,293 @@ __global__ void __launch_bounds__(256) sumsq_partials_kernel(const T* X, uint64_
     const double x = (double)(typename Elem<T>::C)X[j];
     acc = __dadd_rn(acc, __dmul_rn(x, x));
   }
+  return acc;
+}
+
+// Lanes that share a row of `vpr` 16-byte vectors in the row-wise sums: the
+// power of two that covers it (at most 32), so rows are read coalesced.
+__device__ __forceinline__ uint32_t row_lanes(uint32_t vpr) {
+  uint32_t l = 1;
+  while (l < vpr && l < 32) l <<= 1;
+  return l;
+}
+
+// sum_i cnt[i] |X_i|^2 (Nzl2Loss, mf/loss/nzl2.h) over rows dealt to groups of
+// lanes; each lane weighs its own share of a row, four rows in flight.
+template <typename T>
+__device__ __forceinline__ double weighted_squares(const T* X, uint64_t rows, uint32_t rp,
+                                                   const uint32_t* cnt, uint64_t tid,
+                                                   uint64_t stride) {
+  const uint32_t vpr = rp / Elem<T>::VW, lanes = row_lanes(vpr), gl = (uint32_t)tid & (lanes - 1);
+  const uint4* V = reinterpret_cast<const uint4*>(X);
+  const uint64_t groups = stride / lanes;
+  double acc = 0;
+  for (uint64_t i0 = tid / lanes; i0 < rows; i0 += 4 * groups) {
+    for (uint32_t v = gl; v < vpr; v += lanes) {
+      uint4 x[4];
+      double c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint64_t i = i0 + u * groups;
+        x[u] = make_uint4(0, 0, 0, 0);
+        c[u] = 0;
+        if (i < rows) {
+          x[u] = __ldcs(V + i * vpr + v);
+          c[u] = (double)cnt[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc = fma(c[u], add_squares<T>(0.0, x[u]), acc);
+    }
+  }
+  return acc;
+}
+
+// CTAs of 256 threads per SM that the loss kernels' registers are bounded for,
+// by the vector registers a lane holds (N words, V vectors of each side): three
+// at rank 64 or 128 spill (0.58 and 1.12 against 0.55 and 1.05 ms), two at rank
+// 32 leave the SM idle (0.33 against 0.31 ms).
+constexpr int loss_ctas(int N, int V) { return N * V < 16 ? 3 : 2; }
+
+// ---- per-problem (segmented) reductions of the batched form ----------------------
+// One CTA per chunk of a problem's range; owner_sums then adds each problem's
+// chunk partials in chunk order, so every per-problem sum is deterministic.
+template <typename T, int L, int V, int N>
+__global__ void __launch_bounds__(256, loss_ctas(N, V)) nzsl_chunks_kernel(
+    const RangeChunk* chunks, Entries en, const T* W, const T* H, uint32_t r, uint32_t rp,
+    double* partials) {
+  __shared__ double sh[32];
+  const RangeChunk c = chunks[blockIdx.x];
+  const double acc = nzsl_lanes<T, L, V, N>(en, W, H, r, rp, true, c.begin, c.end, threadIdx.x >> 5,
+                                            blockDim.x >> 5);
   const double t = block_reduce(acc, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
-
-template <typename T>
-__device__ __forceinline__ double as_double(T v) { return (double)(float)v; }
-template <>
-__device__ __forceinline__ double as_double<double>(double v) { return v; }
-
-template <typename T>
-__global__ void __launch_bounds__(256) nzl2_partials_kernel(const T* X, uint64_t rows, uint32_t rp,
-                                                            const uint32_t* cnt,
-                                                            double* partials) {
+__global__ void __launch_bounds__(256) nzsl_chunks_exact_kernel(
+    const RangeChunk* chunks, const uint32_t* row, const uint32_t* col, const double* val,
+    const double* W, const double* H, uint32_t r, uint32_t rp, double* partials) {
   __shared__ double sh[32];
-  double acc = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < rows; i += stride) {
-    double v = 0;
-    for (uint32_t z = 0; z < rp; ++z) {
-      const double e = as_double(X[i * rp + z]);
-      v = __dadd_rn(v, __dmul_rn(e, e));
-    }
-    acc = __dadd_rn(acc, __dmul_rn((double)cnt[i], v));
-  }
+  const RangeChunk c = chunks[blockIdx.x];
+  const double acc =
+      nzsl_exact(row, col, val, W, H, r, rp, c.begin + threadIdx.x, c.end, blockDim.x);
   const double t = block_reduce(acc, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) sumsq_chunks_kernel(const RangeChunk* chunks, const T* X,
+                                                           double* partials) {
+  __shared__ double sh[32];
+  const RangeChunk c = chunks[blockIdx.x];  // whole rows or pieces of 2^14 elements: whole vectors
+  const double acc = sum_squares<T>(X + c.begin, c.end - c.begin, threadIdx.x, blockDim.x);
+  const double t = block_reduce(acc, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+}
+__global__ void __launch_bounds__(256) owner_sums_kernel(const double* partials,
+                                                         const uint32_t* owner_begin,
+                                                         double* out) {
+  __shared__ double sh[32];
+  const uint32_t p = blockIdx.x;
+  double acc = 0;
+  for (uint32_t k = owner_begin[p] + threadIdx.x; k < owner_begin[p + 1]; k += blockDim.x)
+    acc = __dadd_rn(acc, partials[k]);
+  const double t = block_reduce(acc, sh);
+  if (threadIdx.x == 0) out[p] = t;
+}
+
+// ---- one launch per loss --------------------------------------------------------
+// Sums of up to K values per thread over the grid: each CTA writes its sums,
+// and the CTA that finishes last adds all CTAs' in a fixed order -- every
+// result is deterministic -- and writes them to `out`, which may be pinned host
+// memory, so a loss is one launch and needs no copy.  MAXK: that value is a
+// maximum instead of a sum.
+template <int K, int MAXK = -1>
+__device__ void grid_sums(double (&v)[K], double* partials, uint32_t* ticket, double* out) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  auto reduce = [&](double x, bool is_max) {
+    const double t = is_max ? block_max(x, sh) : block_reduce(x, sh);
+    __syncthreads();
+    return t;
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double t = reduce(v[k], k == MAXK);
+    if (threadIdx.x == 0) partials[(size_t)k * gridDim.x + blockIdx.x] = t;
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double x = 0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+      const double p = __ldcg(partials + (size_t)k * gridDim.x + i);
+      x = k == MAXK ? fmax(x, p) : __dadd_rn(x, p);
+    }
+    const double t = reduce(x, k == MAXK);
+    if (threadIdx.x == 0) out[k] = t;
+  }
+  if (threadIdx.x == 0) {
+    *ticket = 0;  // for the next launch
+    __threadfence_system();
+  }
+}
+
+// This CTA's share of the loss: the squared errors as v[0], and the terms of
+// the L2 (1) or nonzero-weighted L2 (2) loss of W and of H as v[1], v[2].
+template <typename T>
+__device__ __forceinline__ void loss_terms(const LossArgs& a, double (&v)[3]) {
+  if (a.reg == 0) return;
+  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const T* W = static_cast<const T*>(a.W);
+  const T* H = static_cast<const T*>(a.H);
+  v[1] = a.reg == 1 ? sum_squares<T>(W, a.m * a.rp, tid, stride)
+                    : weighted_squares<T>(W, a.m, a.rp, a.cnt1, tid, stride);
+  v[2] = a.reg == 1 ? sum_squares<T>(H, a.n * a.rp, tid, stride)
+                    : weighted_squares<T>(H, a.n, a.rp, a.cnt2, tid, stride);
+}
+
+__device__ __forceinline__ void loss_finish(const LossArgs& a, double (&v)[3]) {
+  if (a.ticket && a.reg) {
+    grid_sums<3>(v, a.partials, a.ticket, a.out);
+  } else if (a.ticket) {
+    double e[1] = {v[0]};
+    grid_sums<1>(e, a.partials, a.ticket, a.out);
+  } else {
+    __shared__ double sh[32];
+    const double t = block_reduce(v[0], sh);
+    if (threadIdx.x == 0) a.partials[blockIdx.x] = t;
+  }
+}
+
+template <typename T, int L, int V, int N>
+__global__ void __launch_bounds__(256, loss_ctas(N, V)) loss_kernel(LossArgs a) {
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const Entries en{a.row, a.col, static_cast<const float*>(a.val)};
+  double v[3] = {nzsl_lanes<T, L, V, N>(en, static_cast<const T*>(a.W),
+                                        static_cast<const T*>(a.H), a.r, a.rp, a.zero_pad, 0,
+                                        a.nnz, warp, warps), 0, 0};
+  loss_terms<T>(a, v);
+  loss_finish(a, v);
+}
+
+__global__ void __launch_bounds__(256) loss_exact_kernel(LossArgs a) {
+  double v[3] = {nzsl_exact(a.row, a.col, static_cast<const double*>(a.val),
+                            static_cast<const double*>(a.W), static_cast<const double*>(a.H), a.r,
+                            a.rp, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, a.nnz,
+                            (uint64_t)gridDim.x * blockDim.x), 0, 0};
+  loss_terms<double>(a, v);
+  loss_finish(a, v);
+}
+
+// Lanes, vectors per lane and words per vector of the FP32 / BF16 kernels.
+// Rows of whole 32-byte vectors (and bases on 32 bytes) are read with 32-byte
+// loads, others with 16-byte ones; in both, up to 128 bytes of a row per
+// instruction and up to four vectors per lane before more lanes share a row.
+struct LossShape {
+  int lanes, vecs, words;
+};
+LossShape loss_shape(int precision, uint32_t rp, const void* W, const void* H) {
+  const uint32_t bytes = rp * (precision == kFp32 ? 4 : 2);
+  const bool wide = bytes % 32 == 0 &&
+                    ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(H)) & 31u) == 0;
+  LossShape s;
+  s.words = wide ? 8 : 4;
+  const uint32_t nv = bytes / (4 * s.words);
+  s.lanes = nv == 1 ? 1 : nv == 2 && wide ? 2 : 4;
+  while (nv > 4u * s.lanes) s.lanes *= 2;
+  s.vecs = (nv + s.lanes - 1) / s.lanes;
+  return s;
+}
+
+template <typename T>
+void* loss_fn_of(LossShape s, bool chunks) {
+#define DSGDPP_CASE(L, V, N)                                                           \
+  if (s.lanes == L && s.vecs == V && s.words == N)                                     \
+    return chunks ? reinterpret_cast<void*>(&nzsl_chunks_kernel<T, L, V, N>)           \
+                  : reinterpret_cast<void*>(&loss_kernel<T, L, V, N>);
+  DSGDPP_CASE(1, 1, 8) DSGDPP_CASE(2, 1, 8) DSGDPP_CASE(4, 1, 8) DSGDPP_CASE(4, 2, 8)
+  DSGDPP_CASE(4, 3, 8) DSGDPP_CASE(4, 4, 8) DSGDPP_CASE(8, 3, 8) DSGDPP_CASE(8, 4, 8)
+  DSGDPP_CASE(16, 3, 8) DSGDPP_CASE(16, 4, 8)
+  DSGDPP_CASE(1, 1, 4) DSGDPP_CASE(4, 1, 4) DSGDPP_CASE(4, 2, 4) DSGDPP_CASE(4, 3, 4)
+  DSGDPP_CASE(4, 4, 4)
+  DSGDPP_CASE(8, 3, 4) DSGDPP_CASE(8, 4, 4) DSGDPP_CASE(16, 3, 4) DSGDPP_CASE(16, 4, 4)
+  DSGDPP_CASE(32, 3, 4) DSGDPP_CASE(32, 4, 4)
+#undef DSGDPP_CASE
+  return nullptr;
+}
+
+void* loss_fn(int precision, uint32_t rp, const void* W, const void* H, bool chunks) {
+  if (precision == kFp64) return reinterpret_cast<void*>(&loss_exact_kernel);
+  const LossShape s = loss_shape(precision, rp, W, H);
+  return precision == kFp32 ? loss_fn_of<float>(s, chunks) : loss_fn_of<__nv_bfloat16>(s, chunks);
+}
+
+// Sum over rows of |X_i - Xold_i| (v[0]) and their maximum (v[1]): groups of
+// lanes read a row coalesced, two rows in flight.
+template <typename T>
+__device__ __forceinline__ void row_moves(const T* X, const T* Xold, uint64_t rows, uint32_t rp,
+                                          double (&out)[2]) {
+  using C = typename Elem<T>::C;
+  constexpr int VW = Elem<T>::VW;
+  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint32_t vpr = rp / VW, lanes = row_lanes(vpr), gl = (uint32_t)tid & (lanes - 1);
+  const uint64_t groups = (uint64_t)gridDim.x * blockDim.x / lanes;
+  const uint4* A = reinterpret_cast<const uint4*>(X);
+  const uint4* B = reinterpret_cast<const uint4*>(Xold);
+  for (uint64_t k0 = 0; k0 < rows; k0 += 2 * groups) {
+    double s[2] = {0, 0};
+    for (uint32_t v = gl; v < vpr; v += lanes) {
+      uint4 x[2], y[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint64_t i = k0 + u * groups + tid / lanes;
+        x[u] = y[u] = make_uint4(0, 0, 0, 0);
+        if (i < rows) {
+          x[u] = __ldcs(A + i * vpr + v);
+          y[u] = __ldcs(B + i * vpr + v);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        C a[VW], b[VW];
+        Elem<T>::unpack(x[u], a);
+        Elem<T>::unpack(y[u], b);
+#pragma unroll
+        for (int e = 0; e < VW; ++e) {
+          const double d = (double)a[e] - (double)b[e];
+          s[u] += d * d;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      for (uint32_t off = lanes / 2; off > 0; off >>= 1)
+        s[u] += __shfl_xor_sync(kFullMask, s[u], off);
+      if (gl == 0) {
+        const double nrm = sqrt(s[u]);  // rows past the end add 0
+        out[0] += nrm;
+        out[1] = fmax(out[1], nrm);
+      }
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) update_norms_kernel(const T* W, const T* W0, uint64_t m,
+                                                           const T* H, const T* H0, uint64_t n,
+                                                           uint32_t rp, double* partials,
+                                                           uint32_t* ticket, double* out) {
+  double v[2] = {0, 0};
+  row_moves<T>(W, W0, m, rp, v);
+  row_moves<T>(H, H0, n, rp, v);
+  grid_sums<2, 1>(v, partials, ticket, out);
 }
 
 __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partials, uint32_t count,
@@ -391,25 +607,16 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partia
 
 }  // namespace
 
-cudaError_t launch_nzsl_partials(int precision, const uint32_t* row, const uint32_t* col,
-                                 const void* val, uint64_t nnz, const void* W, const void* H,
-                                 uint32_t r, uint32_t rp, double* partials, uint32_t grid,
-                                 cudaStream_t st) {
-  if (precision == kFp64) {
-    nzsl_partials_kernel<double, double><<<grid, 256, 0, st>>>(
-        row, col, (const double*)val, nnz, (const double*)W, (const double*)H, r, rp, partials);
-    return cudaGetLastError();
-  }
-  void* fn = nzsl_fn(precision, rp, false);
+cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st) {
+  void* fn = loss_fn(precision, a.rp, a.W, a.H, false);
   if (!fn) return cudaErrorInvalidValue;
-  const float* v = static_cast<const float*>(val);
-  void* params[] = {&row, &col, &v, &nnz, &W, &H, &r, &rp, &partials};
+  LossArgs args = a;
+  void* params[] = {&args};
   return cudaLaunchKernel(fn, dim3(grid), dim3(256), params, 0, st);
 }
 
-int nzsl_ctas_per_sm(int precision, uint32_t rp) {
-  void* fn = precision == kFp64 ? reinterpret_cast<void*>(&nzsl_partials_kernel<double, double>)
-                                : nzsl_fn(precision, rp, false);
+int loss_ctas_per_sm(int precision, uint32_t rp) {
+  void* fn = loss_fn(precision, rp, nullptr, nullptr, false);
   int n = 0;
   if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 256, 0) != cudaSuccess) return 0;
   return n;
@@ -426,10 +633,10 @@ cudaError_t launch_nzsl_chunks(int precision, const RangeChunk* chunks, uint32_t
                                                       partials);
     return cudaGetLastError();
   }
-  void* fn = nzsl_fn(precision, rp, true);
+  void* fn = loss_fn(precision, rp, W, H, true);
   if (!fn) return cudaErrorInvalidValue;
-  const float* v = static_cast<const float*>(val);
-  void* params[] = {&chunks, &row, &col, &v, &W, &H, &r, &rp, &partials};
+  Entries en{row, col, static_cast<const float*>(val)};
+  void* params[] = {&chunks, &en, &W, &H, &r, &rp, &partials};
   return cudaLaunchKernel(fn, dim3(nchunks), dim3(256), params, 0, st);
 }
 
@@ -453,112 +660,28 @@ cudaError_t launch_owner_sums(const double* partials, const uint32_t* owner_begi
   return cudaGetLastError();
 }
 
-cudaError_t launch_sumsq_partials(int precision, const void* X, uint64_t count,
-                                  double* partials, uint32_t grid, cudaStream_t st) {
-  if (precision == kFp64)
-    sumsq_partials_kernel<double><<<grid, 256, 0, st>>>((const double*)X, count, partials);
-  else if (precision == kFp32)
-    sumsq_partials_kernel<float><<<grid, 256, 0, st>>>((const float*)X, count, partials);
-  else
-    sumsq_partials_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)X, count,
-                                                               partials);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_nzl2_partials(int precision, const void* X, uint64_t rows, uint32_t rp,
-                                 const uint32_t* cnt, double* partials, uint32_t grid,
-                                 cudaStream_t st) {
-  if (precision == kFp64)
-    nzl2_partials_kernel<double><<<grid, 256, 0, st>>>((const double*)X, rows, rp, cnt, partials);
-  else if (precision == kFp32)
-    nzl2_partials_kernel<float><<<grid, 256, 0, st>>>((const float*)X, rows, rp, cnt, partials);
-  else
-    nzl2_partials_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)X, rows, rp,
-                                                              cnt, partials);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_sum_partials(const double* partials, uint32_t count, double* out,
                                 cudaStream_t st) {
   sum_partials_kernel<<<1, 1024, 0, st>>>(partials, count, out);
   return cudaGetLastError();
 }
 
-}  // namespace dsgdpp
-
-// ---- factor-update norms (controller features) -------------------------------------
-namespace dsgdpp {
-namespace {
-
-// Per row: the Euclidean norm of (X - Xold) over the rp entries; per CTA the sum
-// and the maximum of those norms go to partials[blockIdx.x] and
-// partials[gridDim.x + blockIdx.x].
-template <typename T>
-__global__ void __launch_bounds__(256) update_norm_partials_kernel(const T* X, const T* Xold,
-                                                                   uint64_t rows, uint32_t rp,
-                                                                   double* partials) {
-  __shared__ double sh[32];
-  __shared__ double shm[32];
-  double sum = 0, mx = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < rows; i += stride) {
-    double s = 0;
-    for (uint32_t z = 0; z < rp; ++z) {
-      const double dlt = as_double(X[i * rp + z]) - as_double(Xold[i * rp + z]);
-      s += dlt * dlt;
-    }
-    const double nrm = sqrt(s);
-    sum += nrm;
-    mx = fmax(mx, nrm);
-  }
-  const double t = block_reduce(sum, sh);
-  // block max
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(kFullMask, mx, off));
-  if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m2 = 0;
-    for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) m2 = fmax(m2, shm[w]);
-    partials[blockIdx.x] = t;
-    partials[gridDim.x + blockIdx.x] = m2;
-  }
-}
-
-__global__ void max_partials_kernel(const double* partials, uint32_t count, double* out) {
-  __shared__ double sh[32];
-  double mx = 0;
-  for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) mx = fmax(mx, partials[k]);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(kFullMask, mx, off));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m2 = 0;
-    for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) m2 = fmax(m2, sh[w]);
-    out[0] = m2;
-  }
-}
-
-}  // namespace
-
-cudaError_t launch_update_norms(int precision, const void* X, const void* Xold, uint64_t rows,
-                                uint32_t rp, double* partials, uint32_t grid, double* out2,
+cudaError_t launch_update_norms(int precision, const void* W, const void* W0, uint64_t m,
+                                const void* H, const void* H0, uint64_t n, uint32_t rp,
+                                double* partials, uint32_t grid, uint32_t* ticket, double* out,
                                 cudaStream_t st) {
   if (precision == kFp64)
-    update_norm_partials_kernel<double><<<grid, 256, 0, st>>>((const double*)X, (const double*)Xold,
-                                                              rows, rp, partials);
+    update_norms_kernel<double><<<grid, 256, 0, st>>>(
+        (const double*)W, (const double*)W0, m, (const double*)H, (const double*)H0, n, rp,
+        partials, ticket, out);
   else if (precision == kFp32)
-    update_norm_partials_kernel<float><<<grid, 256, 0, st>>>((const float*)X, (const float*)Xold,
-                                                             rows, rp, partials);
+    update_norms_kernel<float><<<grid, 256, 0, st>>>((const float*)W, (const float*)W0, m,
+                                                     (const float*)H, (const float*)H0, n, rp,
+                                                     partials, ticket, out);
   else
-    update_norm_partials_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-        (const __nv_bfloat16*)X, (const __nv_bfloat16*)Xold, rows, rp, partials);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  e = launch_sum_partials(partials, grid, out2, st);
-  if (e != cudaSuccess) return e;
-  max_partials_kernel<<<1, 1024, 0, st>>>(partials + grid, grid, out2 + 1);
+    update_norms_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
+        (const __nv_bfloat16*)W, (const __nv_bfloat16*)W0, m, (const __nv_bfloat16*)H,
+        (const __nv_bfloat16*)H0, n, rp, partials, ticket, out);
   return cudaGetLastError();
 }
 

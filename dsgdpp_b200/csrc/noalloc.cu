@@ -127,9 +127,12 @@ extern "C" int dsgdpp_nzsl_fp32_noalloc(const uint32_t* rows, const uint32_t* co
     if (dsgdpp::launch_sum_partials(scratch, 0, out, st) != cudaSuccess) return DSGDPP_E_CUDA;
     return DSGDPP_OK;
   }
-  if (dsgdpp::launch_nzsl_partials(dsgdpp::kFp32, rows, cols, vals, nnz, W, H, rank, ld, scratch,
-                                   grid, st) != cudaSuccess)
-    return DSGDPP_E_CUDA;
+  dsgdpp::LossArgs a{};
+  a.row = rows; a.col = cols; a.val = vals; a.nnz = nnz;
+  a.W = W; a.H = H;
+  a.r = rank; a.rp = ld;
+  a.partials = scratch;
+  if (dsgdpp::launch_loss(dsgdpp::kFp32, a, grid, st) != cudaSuccess) return DSGDPP_E_CUDA;
   if (dsgdpp::launch_sum_partials(scratch, grid, out, st) != cudaSuccess) return DSGDPP_E_CUDA;
   return DSGDPP_OK;
 }

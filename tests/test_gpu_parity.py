@@ -675,3 +675,39 @@ def test_replay_of_one_column_outlasts_the_round_numbers():
         ref.epoch_explicit(0.001, sched, seeds)
         for a, b in zip(ctx.get_factors(), ref.get_factors()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision,r", [
+    ("fp32", 3), ("fp32", 8), ("fp32", 16), ("fp32", 24), ("fp32", 28), ("fp32", 64),
+    ("fp32", 90), ("fp32", 96), ("fp32", 132), ("fp32", 136), ("fp32", 260), ("fp32", 508),
+    ("fp32", 512), ("bf16", 8), ("bf16", 16), ("bf16", 20), ("bf16", 40), ("bf16", 192),
+    ("bf16", 264), ("bf16", 512), ("bf16", 1016), ("bf16", 1024), ("fp64", 5), ("fp64", 256)])
+@pytest.mark.parametrize("nnz", [1, 31, 4129])
+def test_losses_and_norms_of_every_row_mapping(precision, r, nnz):
+    # against FP64 sums over the stored factors; the sums have at most 4129 r
+    # terms of one sign, so any order of adding them agrees to 1e-12
+    m, n = 70, 61
+    rng = np.random.default_rng(r + nnz)
+    keys = rng.permutation(m * n)[:nnz]
+    rows, cols = (keys // n).astype(np.uint32), (keys % n).astype(np.uint32)
+    vals = rng.standard_normal(nnz)
+    W0, H0 = rng.uniform(-.5, .5, (m, r)), rng.uniform(-.5, .5, (n, r))
+    lanes = 32 if precision == "fp32" and r > 128 else 0  # the epoch kernels' own mapping
+    with P.Context(P.Config(m=m, n=n, rank=r, d=2, precision=precision,
+                            lanes_per_nnz=lanes)) as ctx:
+        ctx.set_matrix(P.TRAIN, rows, cols, vals)
+        ctx.set_factors(W0, H0)
+        W, H = ctx.get_factors()
+        x = vals if precision == "fp64" else vals.astype(np.float32).astype(np.float64)
+        want = float(np.sum((x - np.einsum("ij,ij->i", W[rows], H[cols])) ** 2))
+        w2, h2 = np.sum(W * W, 1), np.sum(H * H, 1)
+        c1, c2 = np.bincount(rows, minlength=m), np.bincount(cols, minlength=n)
+        near = dict(rtol=LOSS_RTOL, atol=0)
+        np.testing.assert_allclose(ctx.nzsl(P.TRAIN), want, **near)
+        np.testing.assert_allclose(ctx.l2(), (w2.sum(), h2.sum()), **near)
+        np.testing.assert_allclose(ctx.nzl2(), (c1 @ w2, c2 @ h2), **near)
+        np.testing.assert_allclose(ctx.loss(), want + w2.sum() + h2.sum(), **near)
+        ctx.save_factors()
+        ctx.set_factors(W0 * 1.5, H0)
+        moved = np.sqrt(np.sum((ctx.get_factors()[0] - W) ** 2, 1))
+        np.testing.assert_allclose(ctx.update_norms(), (moved.sum() / (m + n), moved.max()), **near)

@@ -88,3 +88,22 @@ def test_noalloc_rejects_requests_beyond_capacity():
                                           out.data_ptr(), None) == P.E_INVALID
     assert P.lib.dsgdpp_nzsl_fp32_noalloc(*args, 1, out.data_ptr(), None) == P.OK
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("r,ld,shift", [(30, 32, 0), (30, 32, 4), (32, 32, 4), (8, 16, 0),
+                                        (5, 24, 4), (7, 12, 0), (100, 512, 4)])
+def test_noalloc_leaves_padding_and_alignment_to_the_caller(r, ld, shift):
+    # rows on 16 but not 32 bytes, and a padding that holds anything
+    import torch
+    p = synth.make(300, 200, 2011, 10, rank_true=5, r=r, noise=0.1, seed=r)
+    def rows_of(a):
+        flat = np.full(shift + a.shape[0] * ld, np.nan, np.float32)
+        flat[shift:].reshape(a.shape[0], ld)[:, :r] = a
+        return _device(torch, flat, torch.float32)[shift:]
+    W, H = rows_of(p.W0), rows_of(p.H0)
+    got = _call(torch, _device(torch, p.rows.view(np.int32), torch.int32),
+                _device(torch, p.cols.view(np.int32), torch.int32),
+                _device(torch, p.vals, torch.float32), W, H, r, ld)
+    f = lambda a: a.astype(np.float32).astype(np.float64)
+    want = np.sum((f(p.vals) - np.einsum("ij,ij->i", f(p.W0)[p.rows], f(p.H0)[p.cols])) ** 2)
+    assert got == pytest.approx(float(want), rel=LOSS_RTOL)
