@@ -17,13 +17,16 @@ struct dsgdpp_mlp {
   float* P = nullptr;  // parameters
   float* m = nullptr;  // Adam moments
   float* v = nullptr;
-  float* g = nullptr;  // reduced gradient
-  float* X = nullptr;  // batch buffers (grown on demand)
+  float* partials = nullptr;  // rows of partial gradients (grown on demand)
+  // pinned host memory that the kernels read and write: a batch's inputs,
+  // targets and outputs (grown on demand), the gradient and the loss
+  float* X = nullptr;
   float* Y = nullptr;
   float* out = nullptr;
-  float* grads = nullptr;  // per-sample gradients
-  float* losses = nullptr;
+  float* grad = nullptr;
+  float* loss = nullptr;
   int cap = 0;
+  size_t partials_cap = 0;
   int step = 0;
 };
 
@@ -33,48 +36,43 @@ bool ok(cudaError_t e) { return e == cudaSuccess; }
 
 int grow(dsgdpp_mlp* n, int batch) {
   if (batch <= n->cap) return DSGDPP_OK;
-  const int np = mlp_param_count();
-  cudaFree(n->X); cudaFree(n->Y); cudaFree(n->out); cudaFree(n->grads); cudaFree(n->losses);
-  n->X = n->Y = n->out = n->grads = n->losses = nullptr;
+  for (float** p : {&n->X, &n->Y, &n->out}) {
+    cudaFreeHost(*p);
+    *p = nullptr;
+  }
   n->cap = 0;
-  if (!ok(cudaMalloc(&n->X, (size_t)batch * mlp_input_count() * 4)) ||
-      !ok(cudaMalloc(&n->Y, (size_t)batch * 4)) || !ok(cudaMalloc(&n->out, (size_t)batch * 4)) ||
-      !ok(cudaMalloc(&n->grads, (size_t)batch * np * 4)) ||
-      !ok(cudaMalloc(&n->losses, (size_t)batch * 4)))
+  if (!ok(cudaMallocHost(&n->X, (size_t)batch * mlp_input_count() * 4)) ||
+      !ok(cudaMallocHost(&n->Y, (size_t)batch * 4)) ||
+      !ok(cudaMallocHost(&n->out, (size_t)batch * 4)))
     return DSGDPP_E_NOMEM;
   n->cap = batch;
   return DSGDPP_OK;
 }
 
-int upload(dsgdpp_mlp* n, const float* x, const float* y, int batch) {
+// The batch in the pinned buffers.  Every call below waits for its kernels, so
+// the buffers are free here.
+int stage(dsgdpp_mlp* n, const float* x, const float* y, int batch) {
   if (batch <= 0 || !x) return DSGDPP_E_INVALID;
   if (cudaSetDevice(n->device) != cudaSuccess) return DSGDPP_E_CUDA;
-  int rc = grow(n, batch);
+  const int rc = grow(n, batch);
   if (rc != DSGDPP_OK) return rc;
-  if (!ok(cudaMemcpyAsync(n->X, x, (size_t)batch * mlp_input_count() * 4, cudaMemcpyHostToDevice,
-                          n->stream)))
-    return DSGDPP_E_CUDA;
-  if (y && !ok(cudaMemcpyAsync(n->Y, y, (size_t)batch * 4, cudaMemcpyHostToDevice, n->stream)))
-    return DSGDPP_E_CUDA;
+  std::memcpy(n->X, x, (size_t)batch * mlp_input_count() * 4);
+  if (y) std::memcpy(n->Y, y, (size_t)batch * 4);
   return DSGDPP_OK;
 }
 
-// loss and gradient of the batch already uploaded; sums stay on the device
-int gradient(dsgdpp_mlp* n, int batch, float* loss_out) {
-  if (!ok(launch_mlp(n->P, n->X, n->Y, batch, n->out, n->grads, n->losses, n->stream)) ||
-      !ok(launch_mlp_reduce(n->grads, batch, n->g, n->stream)))
-    return DSGDPP_E_CUDA;
-  if (loss_out) {
-    std::vector<float> l(batch);
-    if (!ok(cudaMemcpyAsync(l.data(), n->losses, (size_t)batch * 4, cudaMemcpyDeviceToHost,
-                            n->stream)) ||
-        !ok(cudaStreamSynchronize(n->stream)))
-      return DSGDPP_E_CUDA;
-    float s = 0;
-    for (float v : l) s += v;
-    *loss_out = s;
+// partial gradients of the staged batch
+int partials(dsgdpp_mlp* n, int batch) {
+  const size_t need = mlp_partials(batch);
+  if (need > n->partials_cap) {
+    cudaFree(n->partials);
+    n->partials = nullptr;
+    n->partials_cap = 0;
+    if (!ok(cudaMalloc(&n->partials, need * 4))) return DSGDPP_E_NOMEM;
+    n->partials_cap = need;
   }
-  return DSGDPP_OK;
+  return ok(launch_mlp(n->P, n->X, n->Y, batch, nullptr, n->partials, n->stream)) ? DSGDPP_OK
+                                                                                  : DSGDPP_E_CUDA;
 }
 
 }  // namespace
@@ -95,7 +93,8 @@ int dsgdpp_mlp_create(int device, uint64_t seed, dsgdpp_mlp** out) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess ||
       !ok(cudaMalloc(&n->P, np * 4)) || !ok(cudaMalloc(&n->m, np * 4)) ||
-      !ok(cudaMalloc(&n->v, np * 4)) || !ok(cudaMalloc(&n->g, np * 4))) {
+      !ok(cudaMalloc(&n->v, np * 4)) || !ok(cudaMallocHost(&n->grad, np * 4)) ||
+      !ok(cudaMallocHost(&n->loss, 4))) {
     dsgdpp_mlp_destroy(n);
     return DSGDPP_E_CUDA;
   }
@@ -122,7 +121,8 @@ void dsgdpp_mlp_destroy(dsgdpp_mlp* n) {
   if (!n) return;
   cudaSetDevice(n->device);
   if (n->stream) cudaStreamSynchronize(n->stream);
-  for (float* p : {n->P, n->m, n->v, n->g, n->X, n->Y, n->out, n->grads, n->losses}) cudaFree(p);
+  for (float* p : {n->P, n->m, n->v, n->partials}) cudaFree(p);
+  for (float* p : {n->X, n->Y, n->out, n->grad, n->loss}) cudaFreeHost(p);
   if (n->stream) cudaStreamDestroy(n->stream);
   delete n;
 }
@@ -148,40 +148,41 @@ int dsgdpp_mlp_set_params(dsgdpp_mlp* n, const float* params) {
 
 int dsgdpp_mlp_forward(dsgdpp_mlp* n, const float* x, int batch, float* out) {
   if (!n || !out) return DSGDPP_E_INVALID;
-  int rc = upload(n, x, nullptr, batch);
+  const int rc = stage(n, x, nullptr, batch);
   if (rc != DSGDPP_OK) return rc;
-  if (!ok(launch_mlp(n->P, n->X, nullptr, batch, n->out, nullptr, nullptr, n->stream)) ||
-      !ok(cudaMemcpyAsync(out, n->out, (size_t)batch * 4, cudaMemcpyDeviceToHost, n->stream)) ||
+  if (!ok(launch_mlp(n->P, n->X, nullptr, batch, n->out, nullptr, n->stream)) ||
       !ok(cudaStreamSynchronize(n->stream)))
     return DSGDPP_E_CUDA;
+  std::memcpy(out, n->out, (size_t)batch * 4);
   return DSGDPP_OK;
 }
 
 int dsgdpp_mlp_gradient(dsgdpp_mlp* n, const float* x, const float* y, int batch, float* loss,
                         float* grad) {
   if (!n || !y) return DSGDPP_E_INVALID;
-  int rc = upload(n, x, y, batch);
+  int rc = stage(n, x, y, batch);
   if (rc != DSGDPP_OK) return rc;
-  rc = gradient(n, batch, loss);
-  if (rc != DSGDPP_OK) return rc;
-  if (grad && (!ok(cudaMemcpyAsync(grad, n->g, mlp_param_count() * 4, cudaMemcpyDeviceToHost,
-                                   n->stream)) ||
-               !ok(cudaStreamSynchronize(n->stream))))
+  if ((rc = partials(n, batch)) != DSGDPP_OK) return rc;
+  if (!ok(launch_mlp_reduce(n->partials, batch, grad ? n->grad : nullptr, n->loss, n->stream)) ||
+      !ok(cudaStreamSynchronize(n->stream)))
     return DSGDPP_E_CUDA;
+  if (loss) *loss = *n->loss;
+  if (grad) std::memcpy(grad, n->grad, mlp_param_count() * 4);
   return DSGDPP_OK;
 }
 
 int dsgdpp_mlp_train_step(dsgdpp_mlp* n, const float* x, const float* y, int batch, float lr,
                           float* loss) {
   if (!n || !y) return DSGDPP_E_INVALID;
-  int rc = upload(n, x, y, batch);
+  int rc = stage(n, x, y, batch);
   if (rc != DSGDPP_OK) return rc;
-  rc = gradient(n, batch, loss);
-  if (rc != DSGDPP_OK) return rc;
+  if ((rc = partials(n, batch)) != DSGDPP_OK) return rc;
   n->step += 1;
-  if (!ok(launch_adam(n->P, n->g, n->m, n->v, lr, 0.9f, 0.999f, 1e-8f, n->step, n->stream)) ||
+  if (!ok(launch_mlp_adam(n->partials, batch, n->loss, n->P, n->m, n->v, lr, 0.9f, 0.999f, 1e-8f,
+                          n->step, n->stream)) ||
       !ok(cudaStreamSynchronize(n->stream)))
     return DSGDPP_E_CUDA;
+  if (loss) *loss = *n->loss;
   return DSGDPP_OK;
 }
 

@@ -197,11 +197,17 @@ cudaError_t launch_update_norms(int precision, const void* W, const void* W0, ui
 // ---- step-size controller network (16 -> 64 -> 64 -> 1, GELU) -----------------------
 int mlp_param_count();
 int mlp_input_count();
+// out (may be null): the clipped outputs; partials (may be null): rows of
+// partial gradients and losses for Y, mlp_partials(batch) floats.  X, Y and out
+// may be pinned host memory, as may grad and loss of the reductions.
+size_t mlp_partials(int batch);
 cudaError_t launch_mlp(const float* P, const float* X, const float* Y, int batch, float* out,
-                       float* grads, float* losses, cudaStream_t st);
-cudaError_t launch_mlp_reduce(const float* grads, int batch, float* grad, cudaStream_t st);
-cudaError_t launch_adam(float* P, const float* g, float* m, float* v, float lr, float b1,
-                        float b2, float eps, int step, cudaStream_t st);
+                       float* partials, cudaStream_t st);
+cudaError_t launch_mlp_reduce(const float* partials, int batch, float* grad, float* loss,
+                              cudaStream_t st);
+cudaError_t launch_mlp_adam(const float* partials, int batch, float* loss, float* P, float* m,
+                            float* v, float lr, float b1, float b2, float eps, int step,
+                            cudaStream_t st);
 
 // ---- data preparation -----------------------------------------------------------
 // The blocking key of an entry is block * stride + its position in the block.

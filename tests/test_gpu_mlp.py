@@ -48,3 +48,24 @@ def test_training_reduces_loss():
     for _ in range(300):
         last = net.train_step(X, y, lr=3e-3)
     assert last < 0.2 * first
+
+
+@pytest.mark.parametrize("batch", [1, 3, 148, 149, 151, 592, 593, 1190])
+def test_batches_that_fill_and_leave_samples_in_the_last_block(batch):
+    # one sample per block up to 148, then four at a time; 64-term FP32 dot
+    # products of values of order 1 err by some 1e-6, tolerances as above
+    net, rng = _net(batch)
+    X = rng.normal(0, 1.0, (batch, 16)).astype(np.float32)
+    y = rng.uniform(-0.9, 0.9, batch).astype(np.float32)
+    want, _ = M.forward(net.params, X)
+    np.testing.assert_allclose(net.forward(X), want, rtol=1e-4, atol=1e-5)
+    loss, g = net.gradient(X, y)
+    wl, wg = M.loss_and_grad(net.params, X, y)
+    assert loss == pytest.approx(wl, rel=1e-4)
+    np.testing.assert_allclose(g, wg, rtol=2e-3, atol=2e-5 * np.max(np.abs(wg)))
+    # a training step moves every parameter against its gradient, by lr at first
+    before = net.params
+    assert net.train_step(X, y, lr=1e-3) == loss
+    moved = net.params - before
+    clear = np.abs(g) > 1e-4
+    np.testing.assert_allclose(moved[clear], -1e-3 * np.sign(g[clear]), rtol=1e-2)
