@@ -23,6 +23,7 @@
 
 #include "../../include/dsgdpp.h"
 #include "context.h"
+#include "hostcopy.h"
 #include "kernels.cuh"
 #include "schedule.h"
 
@@ -107,6 +108,9 @@ struct dsgdpp_batch {
   uint32_t max_chunks = 0;
   uint32_t epoch_counter = 0;
   double epoch_ms = 0;
+  bool holds_pieces = false;    // hostcopy_hold
+  double* staging = nullptr;    // factors on their way to the host, grown on demand
+  size_t staging_cap = 0;
 };
 
 namespace {
@@ -126,13 +130,15 @@ void destroy_impl(dsgdpp_batch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   for (auto& g : b->groups) free_group(g);
   for (void* p : {(void*)b->d_launches, (void*)b->d_segs, (void*)b->d_counters,
-                  (void*)b->d_params, (void*)b->d_partials, (void*)b->d_losses})
+                  (void*)b->d_params, (void*)b->d_partials, (void*)b->d_losses,
+                  (void*)b->staging})
     if (p) cudaFree(p);
   for (void* p : {(void*)b->h_segs, (void*)b->h_params, (void*)b->h_losses})
     if (p) cudaFreeHost(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);
+  if (b->holds_pieces) hostcopy_drop();
 }
 
 // d of a problem: the largest d <= 16 with at least ~2048 entries per block of
@@ -187,6 +193,8 @@ void create_impl(dsgdpp_batch* b, const dsgdpp_config* common, uint32_t count,
                                                             : kLayoutShuffled;
   check_cuda(cudaSetDevice(common->device), "cudaSetDevice");
   check_cuda(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream");
+  hostcopy_hold();
+  b->holds_pieces = true;
   check_cuda(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, common->device),
              "attribute");
   const int prec = common->precision;
@@ -708,16 +716,21 @@ int dsgdpp_batch_get_factors(dsgdpp_batch* b, uint32_t p, double* W, double* H) 
     const Problem& P = b->probs[p];
     const Group& G = b->groups[P.group];
     const size_t es = b->cfg.precision == kFp64 ? 8 : (b->cfg.precision == kFp32 ? 4 : 2);
-    double* tmp = dnew<double>((P.m + P.n) * P.r, "staging");
-    struct F { double* p; ~F() { cudaFree(p); } } f{tmp};
+    const size_t need = (P.m + P.n) * P.r;
+    if (need > b->staging_cap) {
+      dfree(b->staging);
+      b->staging_cap = 0;
+      b->staging = dnew<double>(need, "staging");
+      b->staging_cap = need;
+    }
+    double* tmp = b->staging;
     check_cuda(launch_factor_to_host(b->cfg.precision, (unsigned char*)G.W + P.w0 * G.rp * es,
                                      P.m, P.r, G.rp, tmp, b->stream), "W");
     check_cuda(launch_factor_to_host(b->cfg.precision, (unsigned char*)G.H + P.h0 * G.rp * es,
                                      P.n, P.r, G.rp, tmp + P.m * P.r, b->stream), "H");
-    if (W) check_cuda(cudaMemcpyAsync(W, tmp, P.m * P.r * 8, cudaMemcpyDeviceToHost, b->stream), "D2H");
-    if (H)
-      check_cuda(cudaMemcpyAsync(H, tmp + P.m * P.r, P.n * P.r * 8, cudaMemcpyDeviceToHost,
-                                 b->stream), "D2H");
+    const int dev = b->cfg.device;
+    if (W) check_cuda(copy_to_host(W, tmp, P.m * P.r * 8, dev, b->stream), "D2H");
+    if (H) check_cuda(copy_to_host(H, tmp + P.m * P.r, P.n * P.r * 8, dev, b->stream), "D2H");
     check_cuda(cudaStreamSynchronize(b->stream), "sync");
   });
 }

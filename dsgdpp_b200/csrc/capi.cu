@@ -16,6 +16,7 @@
 
 #include "../../include/dsgdpp.h"
 #include "context.h"
+#include "hostcopy.h"
 #include "rm_device.h"
 #include "kernels.cuh"
 #include "trace_ranges.h"
@@ -149,6 +150,8 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   if (cfg->device < 0 || cfg->device >= ndev) throw Error(DSGDPP_E_CUDA, "no such CUDA device");
   check_cuda(cudaSetDevice(cfg->device), "cudaSetDevice");
   check_cuda(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+  hostcopy_hold();
+  c->holds_pieces = true;
   check_cuda(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, cfg->device),
              "cudaDeviceGetAttribute");
   c->d = cfg->d;
@@ -261,6 +264,7 @@ void destroy_impl(dsgdpp_ctx* c) {
   if (c->ev_vals) cudaEventDestroy(c->ev_vals);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->holds_pieces) hostcopy_drop();
 }
 
 // ---- blocking on the GPU ----------------------------------------------------------
@@ -430,6 +434,7 @@ void set_matrix_impl(dsgdpp_ctx* c, int which, uint64_t nnz, const uint32_t* row
       if (s) cudaStreamSynchronize(s);
     }
   } side_guard;
+  BackgroundCopy vals_copy;  // joined before the guard looks at the stream
   bool vals_on_side = false;
   if (fill) {
     (*fill)(t_rows, t_cols, t_vals, st);
@@ -439,13 +444,12 @@ void set_matrix_impl(dsgdpp_ctx* c, int which, uint64_t nnz, const uint32_t* row
       check_cuda(cudaEventCreateWithFlags(&c->ev_coords, cudaEventDisableTiming), "event");
       check_cuda(cudaEventCreateWithFlags(&c->ev_vals, cudaEventDisableTiming), "event");
     }
-    check_cuda(cudaMemcpyAsync(t_rows, rows, nnz * 4, cudaMemcpyHostToDevice, st), "H2D rows");
-    check_cuda(cudaMemcpyAsync(t_cols, cols, nnz * 4, cudaMemcpyHostToDevice, st), "H2D cols");
+    check_cuda(copy_to_device(t_rows, rows, nnz * 4, c->cfg.device, st), "H2D rows");
+    check_cuda(copy_to_device(t_cols, cols, nnz * 4, c->cfg.device, st), "H2D cols");
     check_cuda(cudaEventRecord(c->ev_coords, st), "event");
     check_cuda(cudaStreamWaitEvent(c->side, c->ev_coords, 0), "wait");
     side_guard.s = c->side;
-    check_cuda(cudaMemcpyAsync(t_vals, vals, nnz * 8, cudaMemcpyHostToDevice, c->side), "H2D vals");
-    check_cuda(cudaEventRecord(c->ev_vals, c->side), "event");
+    vals_copy.start(t_vals, vals, nnz * 8, c->cfg.device, c->side);
     vals_on_side = true;
   }
   check_cuda(cudaMemsetAsync(d_bad, 0, 8, st), "memset");
@@ -503,7 +507,11 @@ void set_matrix_impl(dsgdpp_ctx* c, int which, uint64_t nnz, const uint32_t* row
     check_cuda(launch_count_nnz12(M.row, M.col, u, c->cnt1, c->cnt2, st), "nnz12");
     inverse_counts(c, st);
   }
-  if (vals_on_side) check_cuda(cudaStreamWaitEvent(st, c->ev_vals, 0), "wait values");
+  if (vals_on_side) {
+    check_cuda(vals_copy.join(), "H2D vals");
+    check_cuda(cudaEventRecord(c->ev_vals, c->side), "event");
+    check_cuda(cudaStreamWaitEvent(st, c->ev_vals, 0), "wait values");
+  }
   check_cuda(launch_gather_values(perm, u, head_at, skeys, sidx, nnz, t_vals, M.val, as_double,
                                   st), "gather values");
   check_cuda(cudaStreamSynchronize(st), "sync");
@@ -1026,9 +1034,10 @@ int dsgdpp_set_blocks(dsgdpp_ctx* c, int which, const uint64_t* block_nnz,
       TempDev tmp((nblocks + 1) * 8 + 8);
       uint64_t* d_start = static_cast<uint64_t*>(tmp.p);
       unsigned long long* d_bad = reinterpret_cast<unsigned long long*>(d_start + nblocks + 1);
-      check_cuda(cudaMemcpyAsync(r, local_rows, nnz * 4, cudaMemcpyHostToDevice, st), "H2D rows");
-      check_cuda(cudaMemcpyAsync(col, local_cols, nnz * 4, cudaMemcpyHostToDevice, st), "H2D cols");
-      check_cuda(cudaMemcpyAsync(v, vals, nnz * 8, cudaMemcpyHostToDevice, st), "H2D vals");
+      const int dev = c->cfg.device;
+      check_cuda(copy_to_device(r, local_rows, nnz * 4, dev, st), "H2D rows");
+      check_cuda(copy_to_device(col, local_cols, nnz * 4, dev, st), "H2D cols");
+      check_cuda(copy_to_device(v, vals, nnz * 8, dev, st), "H2D vals");
       check_cuda(cudaMemcpyAsync(d_start, start.data(), (nblocks + 1) * 8, cudaMemcpyHostToDevice,
                                  st), "H2D block starts");
       check_cuda(cudaMemsetAsync(d_bad, 0, 8, st), "memset");
@@ -1125,8 +1134,8 @@ int dsgdpp_set_factors(dsgdpp_ctx* c, const double* W, const double* H) {
     ensure_staging(c);
     const uint64_t m = c->cfg.m, n = c->cfg.n, r = c->r;
     cudaStream_t st = c->stream;
-    check_cuda(cudaMemcpyAsync(c->staging, W, m * r * 8, cudaMemcpyHostToDevice, st), "H2D W");
-    check_cuda(cudaMemcpyAsync(c->staging + m * r, H, n * r * 8, cudaMemcpyHostToDevice, st), "H2D H");
+    check_cuda(copy_to_device(c->staging, W, m * r * 8, c->cfg.device, st), "H2D W");
+    check_cuda(copy_to_device(c->staging + m * r, H, n * r * 8, c->cfg.device, st), "H2D H");
     check_cuda(launch_factor_to_device(c->cfg.precision, c->staging, m, c->r, c->rp, c->W, st), "W");
     check_cuda(launch_factor_to_device(c->cfg.precision, c->staging + m * r, n, c->r, c->rp, c->H,
                                        st), "H");
@@ -1145,10 +1154,8 @@ int dsgdpp_get_factors(dsgdpp_ctx* c, double* W, double* H) {
     check_cuda(launch_factor_to_host(c->cfg.precision, c->W, m, c->r, c->rp, c->staging, st), "W");
     check_cuda(launch_factor_to_host(c->cfg.precision, c->H, n, c->r, c->rp, c->staging + m * r,
                                      st), "H");
-    if (W) check_cuda(cudaMemcpyAsync(W, c->staging, m * r * 8, cudaMemcpyDeviceToHost, st), "D2H W");
-    if (H)
-      check_cuda(cudaMemcpyAsync(H, c->staging + m * r, n * r * 8, cudaMemcpyDeviceToHost, st),
-                 "D2H H");
+    if (W) check_cuda(copy_to_host(W, c->staging, m * r * 8, c->cfg.device, st), "D2H W");
+    if (H) check_cuda(copy_to_host(H, c->staging + m * r, n * r * 8, c->cfg.device, st), "D2H H");
     check_cuda(cudaStreamSynchronize(st), "sync");
     return DSGDPP_OK;
   });

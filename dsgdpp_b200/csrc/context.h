@@ -89,6 +89,7 @@ struct dsgdpp_ctx {
   uint32_t* cnt2 = nullptr;
   void* inv1 = nullptr;
   void* inv2 = nullptr;
+  bool holds_pieces = false;  // hostcopy_hold
   double* staging = nullptr;  // (m + n) * r doubles, factor upload / download
   void* scratch = nullptr;    // blocking scratch of set_matrix, grown on demand
   size_t scratch_bytes = 0;

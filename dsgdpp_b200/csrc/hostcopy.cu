@@ -1,0 +1,216 @@
+// hostcopy.cu -- see hostcopy.h.
+#include "hostcopy.h"
+
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+#include <system_error>
+#include <vector>
+
+namespace dsgdpp {
+namespace {
+
+// Measured on a B200 host with 16 cores, 358 MB of factors to the device / back:
+// 32 / 75 ms through the driver, 8.6 / 16 ms in pieces of 1 MB, 12.5 / 20 ms in
+// pieces of 512 KB.
+constexpr size_t kPiece = 1 << 20;
+constexpr size_t kDirect = 2 << 20;  // below this the driver's own path is as fast
+constexpr unsigned kThreads = 8;
+// One slab serves one copy.  Page-locking it costs some 7 ms, what the pieces
+// save on about 90 MB, so the first is made once that much has been copied
+// (a program that loads little never pays for it).
+constexpr size_t kSlabPieces = 2 * kThreads;
+constexpr size_t kMaxSlabs = 2;  // 32 MB
+constexpr size_t kSlabAfter = 64 << 20;
+
+std::mutex g_mutex;
+std::vector<void*> g_slabs;
+std::vector<void*> g_free;  // pieces not in use
+size_t g_holders = 0;
+size_t g_copied = 0;        // bytes copied directly since there was no slab
+
+void free_slabs_if_unused() {  // under the mutex
+  if (g_slabs.empty() || g_holders > 0 || g_free.size() != g_slabs.size() * kSlabPieces) return;
+  for (void* p : g_slabs) cudaFreeHost(p);
+  g_slabs.clear();
+  g_free.clear();
+  g_copied = 0;
+}
+
+bool worth_staging(size_t bytes) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (!g_slabs.empty()) return true;
+  g_copied += bytes;
+  return g_copied >= kSlabAfter;
+}
+
+void* take_piece() {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (g_free.empty()) {
+    if (g_slabs.size() >= kMaxSlabs) return nullptr;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kPiece * kSlabPieces, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();  // not an error of the copy: it goes the direct way
+      return nullptr;
+    }
+    g_slabs.push_back(p);
+    for (size_t k = kSlabPieces; k-- > 0;) g_free.push_back(static_cast<char*>(p) + k * kPiece);
+  }
+  void* p = g_free.back();
+  g_free.pop_back();
+  return p;
+}
+
+void give_piece(void* p) {
+  if (!p) return;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  g_free.push_back(p);
+  free_slabs_if_unused();
+}
+
+bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type != cudaMemoryTypeUnregistered;
+}
+
+// One worker: pieces first, first + step, ... of the copy through two
+// page-locked pieces of its own, one travelling while the other is filled or
+// emptied.  Without pieces (none to be had) it copies directly.
+cudaError_t work(char* dst, const char* src, size_t bytes, size_t first, size_t step, bool to_host,
+                 int device, cudaStream_t st) {
+  cudaError_t e = cudaSetDevice(device);
+  if (e != cudaSuccess) return e;
+  struct Slot {
+    void* p = nullptr;
+    cudaEvent_t done = nullptr;
+    size_t at = 0, len = 0;  // the piece of the copy it holds (to_host)
+    bool busy = false;
+  } slot[2];
+  for (Slot& s : slot) {
+    s.p = take_piece();
+    if (cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess) s.done = nullptr;
+  }
+  const bool staged = slot[0].p && slot[1].p && slot[0].done && slot[1].done;
+  auto finish = [&](Slot& s) {  // the slot's transfer is over; hand out what it brought
+    if (!s.busy) return cudaSuccess;
+    s.busy = false;
+    const cudaError_t r = cudaEventSynchronize(s.done);
+    if (r == cudaSuccess && to_host) std::memcpy(dst + s.at, s.p, s.len);
+    return r;
+  };
+  int k = 0;
+  for (size_t at = first * kPiece; at < bytes && e == cudaSuccess; at += step * kPiece, k ^= 1) {
+    const size_t len = std::min(kPiece, bytes - at);
+    if (!staged) {
+      e = cudaMemcpyAsync(dst + at, src + at, len,
+                          to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
+      continue;
+    }
+    Slot& s = slot[k];
+    e = finish(s);
+    if (e != cudaSuccess) break;
+    if (to_host) {
+      e = cudaMemcpyAsync(s.p, src + at, len, cudaMemcpyDeviceToHost, st);
+    } else {
+      std::memcpy(s.p, src + at, len);
+      e = cudaMemcpyAsync(dst + at, s.p, len, cudaMemcpyHostToDevice, st);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(s.done, st);
+    s.at = at;
+    s.len = len;
+    s.busy = e == cudaSuccess;
+  }
+  for (int j = 0; j < 2; ++j) {  // in the order they were started
+    const cudaError_t r = finish(slot[k ^ j]);
+    if (e == cudaSuccess) e = r;
+  }
+  if (!staged && to_host && e == cudaSuccess) e = cudaStreamSynchronize(st);
+  // after a failure a transfer may still use the pieces
+  if (e != cudaSuccess) cudaStreamSynchronize(st);
+  for (Slot& s : slot) {
+    give_piece(s.p);
+    if (s.done) cudaEventDestroy(s.done);
+  }
+  return e;
+}
+
+cudaError_t copy(void* dst, const void* src, size_t bytes, bool to_host, int device,
+                 cudaStream_t st) {
+  if (bytes == 0) return cudaSuccess;
+  const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+  const void* host = to_host ? dst : src;
+  if (bytes < kDirect || page_locked(host) || !worth_staging(bytes))
+    return cudaMemcpyAsync(dst, src, bytes, kind, st);
+  const size_t pieces = (bytes + kPiece - 1) / kPiece;
+  const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+  const unsigned n = (unsigned)std::min<size_t>({kThreads, cores, (pieces + 1) / 2});
+  cudaError_t status[kThreads];
+  std::thread pool[kThreads];
+  auto one = [&](unsigned t) {
+    status[t] = work(static_cast<char*>(dst), static_cast<const char*>(src), bytes, t, n, to_host,
+                     device, st);
+  };
+  unsigned started = 1;
+  for (; started < n; ++started) {
+    try {
+      pool[started] = std::thread(one, started);
+    } catch (const std::system_error&) {
+      break;  // no more threads: this one does the rest
+    }
+  }
+  one(0);
+  for (unsigned t = started; t < n; ++t) one(t);
+  for (unsigned t = 1; t < started; ++t) pool[t].join();
+  for (unsigned t = 0; t < n; ++t)
+    if (status[t] != cudaSuccess) return status[t];
+  return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t copy_to_device(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
+  return copy(dst, src, bytes, false, device, st);
+}
+
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
+  return copy(dst, src, bytes, true, device, st);
+}
+
+void BackgroundCopy::start(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
+  join();
+  auto run = [this, dst, src, bytes, device, st]() {
+    status_ = cudaSetDevice(device);
+    if (status_ == cudaSuccess) status_ = copy_to_device(dst, src, bytes, device, st);
+  };
+  if (bytes < kDirect || page_locked(src)) {
+    run();
+    return;
+  }
+  try {
+    thread_ = std::thread(run);
+  } catch (const std::system_error&) {
+    run();
+  }
+}
+
+cudaError_t BackgroundCopy::join() {
+  if (thread_.joinable()) thread_.join();
+  return status_;
+}
+
+void hostcopy_hold() {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  ++g_holders;
+}
+
+void hostcopy_drop() {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  --g_holders;
+  free_slabs_if_unused();
+}
+
+}  // namespace dsgdpp

@@ -711,3 +711,50 @@ def test_losses_and_norms_of_every_row_mapping(precision, r, nnz):
         ctx.set_factors(W0 * 1.5, H0)
         moved = np.sqrt(np.sum((ctx.get_factors()[0] - W) ** 2, 1))
         np.testing.assert_allclose(ctx.update_norms(), (moved.sum() / (m + n), moved.max()), **near)
+
+
+@pytest.mark.parametrize("m,n,r", [(26214, 26215, 10), (131072, 3, 2), (131073, 200, 2),
+                                   (400001, 300007, 3), (1000, 900, 700)])
+def test_factors_through_pageable_and_page_locked_arrays(m, n, r):
+    # 2 MiB - 32 bytes (copied as they are), exactly 2 MiB, a byte count just
+    # above, and many pieces with an odd end
+    import torch
+    rng = np.random.default_rng(m)
+    W0, H0 = rng.standard_normal((m, r)), rng.standard_normal((n, r))
+    lanes = 32 if r > 256 else 0
+    with P.Context(P.Config(m=m, n=n, rank=min(r, 256), d=1, precision="fp64",
+                            lanes_per_nnz=lanes)) as ctx:
+        W0, H0 = W0[:, :256].copy(), H0[:, :256].copy()
+        for lock in (False, True):
+            give = (lambda a: torch.from_numpy(a).pin_memory().numpy()) if lock else np.copy
+            ctx.set_factors(give(W0), give(H0))
+            W, H = ctx.get_factors()
+            np.testing.assert_array_equal(W, W0)
+            np.testing.assert_array_equal(H, H0)
+            W, H = give(np.zeros_like(W0)), give(np.zeros_like(H0))
+            ctx.get_factors_into(W, H)
+            np.testing.assert_array_equal(W, W0)
+            np.testing.assert_array_equal(H, H0)
+
+
+@pytest.mark.parametrize("nnz", [200_000, 262_144, 524_289, 1_300_001])
+def test_matrix_from_pageable_and_page_locked_arrays(nnz):
+    import torch
+    rng = np.random.default_rng(nnz)
+    rows = rng.integers(0, 5000, nnz).astype(np.uint32)  # some pairs repeat: values are summed
+    cols = rng.integers(0, 4000, nnz).astype(np.uint32)
+    vals = rng.standard_normal(nnz)
+    lock = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a
+                                      ).pin_memory().numpy().view(a.dtype)
+    got = []
+    for give in (np.copy, lock):
+        with P.Context(P.Config(m=5000, n=4000, rank=4, d=3, precision="fp64")) as ctx:
+            ctx.set_matrix(P.TRAIN, give(rows), give(cols), give(vals))
+            ctx.set_factors(np.zeros((5000, 4)), np.zeros((4000, 4)))
+            got.append((ctx.block_nnz(), *ctx.nnz12()[:2], ctx.nzsl(P.TRAIN)))
+            bad = rows.copy()
+            bad[nnz // 2] = 5000  # refused while the values are still on their way
+            with pytest.raises(P.DsgdppError):
+                ctx.set_matrix(P.TRAIN, give(bad), give(cols), give(vals))
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
