@@ -546,12 +546,19 @@ void losses(dsgdpp_batch* b, bool test) {
     // tables in group order; write them to a group-local area, then scatter
     const uint32_t np = (uint32_t)G.probs.size();
     double* out = b->d_losses;  // [4][np] for this group, reused per group
-    check_cuda(launch_nzsl_chunks(prec, G.d_nchunks, G.nn, G.row, G.col, G.val, G.W, G.H, G.rp,
-                                  G.rp, b->d_partials, st), "loss");
+    LossArgs a{};
+    a.row = G.row; a.col = G.col; a.val = G.val;
+    a.W = G.W; a.H = G.H;
+    a.r = a.rp = G.rp;
+    a.zero_pad = true;
+    a.partials = b->d_partials;
+    a.chunks = G.d_nchunks;
+    if (G.nn) check_cuda(launch_loss(prec, a, G.nn, st), "loss");
     check_cuda(launch_owner_sums(b->d_partials, G.d_nown, np, out, st), "loss");
     if (test) {
-      check_cuda(launch_nzsl_chunks(prec, G.d_tchunks, G.nt, G.trow, G.tcol, G.tval, G.W, G.H,
-                                    G.rp, G.rp, b->d_partials, st), "test loss");
+      a.row = G.trow; a.col = G.tcol; a.val = G.tval;
+      a.chunks = G.d_tchunks;
+      if (G.nt) check_cuda(launch_loss(prec, a, G.nt, st), "test loss");
       check_cuda(launch_owner_sums(b->d_partials, G.d_town, np, out + np, st), "test loss");
     }
     check_cuda(launch_sumsq_chunks(prec, G.d_wchunks, G.nw, G.W, b->d_partials, st), "l2");

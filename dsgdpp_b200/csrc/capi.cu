@@ -205,7 +205,7 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   c->d_mask = dalloc<uint8_t>((size_t)d2 * d2, "mask");
   // one resident wave of the loss kernel; fixed per context, so every loss
   // of the context is reduced in the same order
-  const int loss_per_sm = loss_ctas_per_sm(cfg->precision, c->rp);
+  const int loss_per_sm = loss_ctas_per_sm(cfg->precision, c->r, c->rp);
   c->loss_grid = (uint32_t)c->num_sms * (uint32_t)std::max(2, std::min(8, loss_per_sm));
   c->d_partials = dalloc<double>(3 * (size_t)c->loss_grid, "partials");
   c->d_loss_ticket = dalloc<uint32_t>(1, "loss ticket");

@@ -141,6 +141,11 @@ cudaError_t launch_scale_rows(int precision, void* W, uint64_t wrows, void* H, u
                               uint32_t rp, const uint32_t* w_slot, const uint32_t* h_slot,
                               const float* scales, cudaStream_t st);
 
+// A range of entries or factor elements.
+struct RangeChunk {
+  uint64_t begin, end;
+};
+
 // A loss in one launch: the squared errors of the entries, and with `reg` the
 // sums of squares of W and H (1) or their count-weighted forms (2).  With a
 // ticket (a zeroed word that the launch leaves zeroed) out[0 .. 2] (out[0]
@@ -156,31 +161,25 @@ struct LossArgs {
   const void* H;
   uint64_t m, n;
   uint32_t r, rp;
-  bool zero_pad;         // rows hold zeros from r to rp (FP32 / BF16)
+  bool zero_pad;         // rows hold zeros from r to rp (may be false for FP32)
   int reg;
   const uint32_t* cnt1;  // reg 2: nnz1, nnz2
   const uint32_t* cnt2;
+  const RangeChunk* chunks;  // squared errors of these ranges, one per CTA (no ticket)
   double* partials;
   uint32_t* ticket;
   double* out;
 };
 cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st);
-// CTAs per SM of the loss kernel for this precision and row width
-int loss_ctas_per_sm(int precision, uint32_t rp);
+// CTAs per SM of the loss kernel for this precision, rank and row width
+int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp);
 // out[0] = the sum of `count` partials
 cudaError_t launch_sum_partials(const double* partials, uint32_t count, double* out,
                                 cudaStream_t st);
 
 // Per-problem sums of the batched form: one CTA per range chunk writes
-// partials[chunk]; owner_sums adds partials[owner_begin[p] .. owner_begin[p+1])
+// partials[chunk] (LossArgs::chunks, sumsq_chunks); owner_sums adds partials[owner_begin[p] .. owner_begin[p+1])
 // in order into out[p] for p < owners.
-struct RangeChunk {
-  uint64_t begin, end;
-};
-cudaError_t launch_nzsl_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
-                               const uint32_t* row, const uint32_t* col, const void* val,
-                               const void* W, const void* H, uint32_t r, uint32_t rp,
-                               double* partials, cudaStream_t st);
 cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
                                 const void* X, double* partials, cudaStream_t st);
 cudaError_t launch_owner_sums(const double* partials, const uint32_t* owner_begin,

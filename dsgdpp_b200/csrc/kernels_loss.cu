@@ -106,27 +106,26 @@ __device__ __forceinline__ uint32_t elem_bits(const Words<N>& v, int e) {
 // at BF16 rank 32; 32 spill, or halve the warps)
 constexpr int kLossWords = 16;
 
-struct Entries {
-  const uint32_t* row;
-  const uint32_t* col;
-  const float* val;
-};
-
-// The squared error of 32 entries (nrec of them exist), one entry per lane in
-// the end.  FAST: all 32 exist and rows are padded with zeros, so whole vectors
-// are summed; a lane past the row's end reads its first vector and drops it.
-template <typename T, int L, int V, int N, bool FAST>
+// The squared error of 32 entries (nrec of them exist; the others name rows
+// that exist), one entry per lane in the end.  A lane whose vector starts past
+// the rank reads the row's first one and drops it; with MASK a vector that
+// reaches past the rank is masked there (rows whose padding is not zero).
+template <typename T, int L, int V, int N, bool MASK>
 __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, float my_val,
                                             uint32_t nrec, const T* W, const T* H, uint32_t r,
                                             uint32_t rp) {
-  constexpr int NG = 32 / L;                       // entries per round
-  constexpr int EPV = N * 4 / (int)sizeof(T);      // elements per vector
+  constexpr int NG = 32 / L;                   // entries per round
+  constexpr int EPV = N * 4 / (int)sizeof(T);  // elements per vector
   // vectors of each side that a lane has in flight: U rounds of a row's V, or
   // C of one round's
   constexpr int F = kLossWords / N;
   constexpr int C = V < F ? V : F;
   constexpr int U = F / V < 1 ? 1 : F / V < L ? F / V : L;
   const uint32_t lane = threadIdx.x & 31u, grp = lane / L, gl = lane % L;
+  // this lane's last vector: only it may start past the rank, or reach past it
+  const uint32_t z_last = (uint32_t)((V - 1) * L + gl) * EPV;
+  const bool last_in = z_last < r;
+  const uint32_t last_at = last_in ? z_last : 0;
   double ip[L];
 #pragma unroll
   for (int t0 = 0; t0 < L; t0 += U) {
@@ -144,19 +143,9 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (v0 + c >= V) continue;
-          const uint32_t z0 = (uint32_t)((v0 + c) * L + gl) * EPV;
-          if constexpr (FAST) {
-            const uint32_t at = v0 + c < V - 1 || z0 < rp ? z0 : 0;  // only the last may not exist
-            wv[u][c] = load_words<N>(w + at);
-            hv[u][c] = load_words<N>(h + at);
-          } else {
-            wv[u][c] = Words<N>{};
-            hv[u][c] = Words<N>{};
-            if (ri < nrec && z0 < rp) {
-              wv[u][c] = load_words<N>(w + z0);
-              hv[u][c] = load_words<N>(h + z0);
-            }
-          }
+          const uint32_t at = v0 + c == V - 1 ? last_at : (uint32_t)((v0 + c) * L + gl) * EPV;
+          wv[u][c] = load_words<N>(w + at);
+          hv[u][c] = load_words<N>(h + at);
         }
       }
 #pragma unroll
@@ -165,27 +154,28 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (v0 + c >= V) continue;
-          const uint32_t z0 = (uint32_t)((v0 + c) * L + gl) * EPV;
+          if (MASK && v0 + c == V - 1) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+              // whole words past the rank, and the upper half of one that ends it
+              const uint32_t z = z_last + k * (4 / (uint32_t)sizeof(T));
+              const uint32_t keep = z >= r ? 0u : z + 4 / (uint32_t)sizeof(T) > r ? 0xffffu : ~0u;
+              wv[u][c].w[k] &= keep;
+              hv[u][c].w[k] &= keep;
+            }
+          }
+          const double before = s;
           // The product of two floats is exact in FP64, so the fused
           // multiply-add rounds exactly like the separate add.  The sum is
           // formed with H scaled by 2^-896 and scaled back once: a power of
           // two, so it rounds exactly as unscaled wherever the scaled terms
           // stay normal doubles (magnitudes of 2^-126 and up; below that the
           // absolute error stays under 2^-178).
-          if (FAST || z0 + EPV <= r) {
-            const double before = s;
 #pragma unroll
-            for (int e = 0; e < EPV; ++e)
-              s = fma((double)__uint_as_float(elem_bits<T>(wv[u][c], e)),
-                      f32_scaled(elem_bits<T>(hv[u][c], e)), s);
-            if (FAST && v0 + c == V - 1 && z0 >= rp) s = before;
-          } else {
-#pragma unroll
-            for (int e = 0; e < EPV; ++e)
-              if (z0 + e < r)
-                s = fma((double)__uint_as_float(elem_bits<T>(wv[u][c], e)),
-                        f32_scaled(elem_bits<T>(hv[u][c], e)), s);
-          }
+          for (int e = 0; e < EPV; ++e)
+            s = fma((double)__uint_as_float(elem_bits<T>(wv[u][c], e)),
+                    f32_scaled(elem_bits<T>(hv[u][c], e)), s);
+          if (v0 + c == V - 1 && !last_in) s = before;
         }
         ip[t0 + u] = s;
       }
@@ -204,23 +194,25 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
   const uint32_t ri = gl * NG + grp;
   const float x = __shfl_sync(kFullMask, my_val, ri);
   const double diff = __dsub_rn((double)x, __dmul_rn(ip[0], 0x1p896));
-  return FAST || ri < nrec ? __dmul_rn(diff, diff) : 0.0;
+  return ri < nrec ? __dmul_rn(diff, diff) : 0.0;
 }
 
 // Entries [begin, end) dealt to warps warp, warp + nwarps, ... 32 at a time.
-template <typename T, int L, int V, int N>
-__device__ __forceinline__ double nzsl_lanes(const Entries& en, const T* W, const T* H, uint32_t r,
-                                             uint32_t rp, bool zero_pad, uint64_t begin,
-                                             uint64_t end, uint64_t warp, uint64_t nwarps) {
+template <typename T, int L, int V, int N, bool MASK>
+__device__ __forceinline__ double nzsl_lanes(const LossArgs& a, uint64_t begin, uint64_t end,
+                                             uint64_t warp, uint64_t nwarps) {
   const uint32_t lane = threadIdx.x & 31u;
+  const T* W = static_cast<const T*>(a.W);
+  const T* H = static_cast<const T*>(a.H);
+  const float* val = static_cast<const float*>(a.val);
   double acc = 0;
   uint64_t base = begin + warp * 32;
-  uint32_t n_row = 0, n_col = 0;
+  uint32_t n_row = 0, n_col = 0;  // of a lane without an entry: row 0, or an earlier entry's
   float n_val = 0;
   if (base + lane < end) {
-    n_row = en.row[base + lane];
-    n_col = en.col[base + lane];
-    n_val = en.val[base + lane];
+    n_row = a.row[base + lane];
+    n_col = a.col[base + lane];
+    n_val = val[base + lane];
   }
   for (; base < end; base += nwarps * 32) {
     const uint32_t my_row = n_row, my_col = n_col;
@@ -228,15 +220,13 @@ __device__ __forceinline__ double nzsl_lanes(const Entries& en, const T* W, cons
     // the next 32 entries travel while these are summed
     const uint64_t nk = base + nwarps * 32 + lane;
     if (nk < end) {
-      n_row = en.row[nk];
-      n_col = en.col[nk];
-      n_val = en.val[nk];
+      n_row = a.row[nk];
+      n_col = a.col[nk];
+      n_val = val[nk];
     }
     const uint32_t nrec = (uint32_t)min((uint64_t)32, end - base);
-    acc = __dadd_rn(acc, nrec == 32 && zero_pad
-                             ? squares32<T, L, V, N, true>(my_row, my_col, my_val, nrec, W, H, r, rp)
-                             : squares32<T, L, V, N, false>(my_row, my_col, my_val, nrec, W, H, r,
-                                                            rp));
+    acc = __dadd_rn(acc, squares32<T, L, V, N, MASK>(my_row, my_col, my_val, nrec, W, H, a.r,
+                                                     a.rp));
   }
   return acc;
 }
@@ -358,27 +348,6 @@ constexpr int loss_ctas(int N, int V) { return N * V < 16 ? 3 : 2; }
 // ---- per-problem (segmented) reductions of the batched form ----------------------
 // One CTA per chunk of a problem's range; owner_sums then adds each problem's
 // chunk partials in chunk order, so every per-problem sum is deterministic.
-template <typename T, int L, int V, int N>
-__global__ void __launch_bounds__(256, loss_ctas(N, V)) nzsl_chunks_kernel(
-    const RangeChunk* chunks, Entries en, const T* W, const T* H, uint32_t r, uint32_t rp,
-    double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  const double acc = nzsl_lanes<T, L, V, N>(en, W, H, r, rp, true, c.begin, c.end, threadIdx.x >> 5,
-                                            blockDim.x >> 5);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
-__global__ void __launch_bounds__(256) nzsl_chunks_exact_kernel(
-    const RangeChunk* chunks, const uint32_t* row, const uint32_t* col, const double* val,
-    const double* W, const double* H, uint32_t r, uint32_t rp, double* partials) {
-  __shared__ double sh[32];
-  const RangeChunk c = chunks[blockIdx.x];
-  const double acc =
-      nzsl_exact(row, col, val, W, H, r, rp, c.begin + threadIdx.x, c.end, blockDim.x);
-  const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t;
-}
 template <typename T>
 __global__ void __launch_bounds__(256) sumsq_chunks_kernel(const RangeChunk* chunks, const T* X,
                                                            double* partials) {
@@ -471,24 +440,37 @@ __device__ __forceinline__ void loss_finish(const LossArgs& a, double (&v)[3]) {
   }
 }
 
-template <typename T, int L, int V, int N>
+template <typename T, int L, int V, int N, bool MASK>
 __global__ void __launch_bounds__(256, loss_ctas(N, V)) loss_kernel(LossArgs a) {
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const Entries en{a.row, a.col, static_cast<const float*>(a.val)};
-  double v[3] = {nzsl_lanes<T, L, V, N>(en, static_cast<const T*>(a.W),
-                                        static_cast<const T*>(a.H), a.r, a.rp, a.zero_pad, 0,
-                                        a.nnz, warp, warps), 0, 0};
-  loss_terms<T>(a, v);
+  const uint32_t per = blockDim.x >> 5, w = threadIdx.x >> 5;
+  // entries [begin, end): of the whole grid, or of CTA k in range k
+  uint64_t begin = 0, end = a.nnz, warp = (uint64_t)blockIdx.x * per + w;
+  uint64_t nwarps = (uint64_t)gridDim.x * per;
+  if (a.chunks) {
+    begin = a.chunks[blockIdx.x].begin;
+    end = a.chunks[blockIdx.x].end;
+    warp = w;
+    nwarps = per;
+  }
+  double v[3] = {nzsl_lanes<T, L, V, N, MASK>(a, begin, end, warp, nwarps), 0, 0};
+  if (!a.chunks) loss_terms<T>(a, v);
   loss_finish(a, v);
 }
 
 __global__ void __launch_bounds__(256) loss_exact_kernel(LossArgs a) {
-  double v[3] = {nzsl_exact(a.row, a.col, static_cast<const double*>(a.val),
-                            static_cast<const double*>(a.W), static_cast<const double*>(a.H), a.r,
-                            a.rp, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, a.nnz,
-                            (uint64_t)gridDim.x * blockDim.x), 0, 0};
-  loss_terms<double>(a, v);
+  double v[3] = {0, 0, 0};
+  uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, end = a.nnz;
+  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  if (a.chunks) {
+    const RangeChunk c = a.chunks[blockIdx.x];
+    first = c.begin + threadIdx.x;
+    end = c.end;
+    stride = blockDim.x;
+  }
+  v[0] = nzsl_exact(a.row, a.col, static_cast<const double*>(a.val),
+                    static_cast<const double*>(a.W), static_cast<const double*>(a.H), a.r, a.rp,
+                    first, end, stride);
+  if (!a.chunks) loss_terms<double>(a, v);
   loss_finish(a, v);
 }
 
@@ -499,25 +481,24 @@ __global__ void __launch_bounds__(256) loss_exact_kernel(LossArgs a) {
 struct LossShape {
   int lanes, vecs, words;
 };
-LossShape loss_shape(int precision, uint32_t rp, const void* W, const void* H) {
-  const uint32_t bytes = rp * (precision == kFp32 ? 4 : 2);
-  const bool wide = bytes % 32 == 0 &&
+LossShape loss_shape(int precision, uint32_t r, uint32_t rp, const void* W, const void* H) {
+  const uint32_t es = precision == kFp32 ? 4 : 2;
+  const bool wide = rp * es % 32 == 0 &&
                     ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(H)) & 31u) == 0;
   LossShape s;
   s.words = wide ? 8 : 4;
-  const uint32_t nv = bytes / (4 * s.words);
+  const uint32_t nv = (r * es + 4 * s.words - 1) / (4 * s.words);  // vectors up to the rank
   s.lanes = nv == 1 ? 1 : nv == 2 && wide ? 2 : 4;
   while (nv > 4u * s.lanes) s.lanes *= 2;
   s.vecs = (nv + s.lanes - 1) / s.lanes;
   return s;
 }
 
-template <typename T>
-void* loss_fn_of(LossShape s, bool chunks) {
-#define DSGDPP_CASE(L, V, N)                                                           \
-  if (s.lanes == L && s.vecs == V && s.words == N)                                     \
-    return chunks ? reinterpret_cast<void*>(&nzsl_chunks_kernel<T, L, V, N>)           \
-                  : reinterpret_cast<void*>(&loss_kernel<T, L, V, N>);
+template <typename T, bool MASK>
+void* loss_fn_of(LossShape s) {
+#define DSGDPP_CASE(L, V, N) \
+  if (s.lanes == L && s.vecs == V && s.words == N) \
+    return reinterpret_cast<void*>(&loss_kernel<T, L, V, N, MASK>);
   DSGDPP_CASE(1, 1, 8) DSGDPP_CASE(2, 1, 8) DSGDPP_CASE(4, 1, 8) DSGDPP_CASE(4, 2, 8)
   DSGDPP_CASE(4, 3, 8) DSGDPP_CASE(4, 4, 8) DSGDPP_CASE(8, 3, 8) DSGDPP_CASE(8, 4, 8)
   DSGDPP_CASE(16, 3, 8) DSGDPP_CASE(16, 4, 8)
@@ -529,10 +510,12 @@ void* loss_fn_of(LossShape s, bool chunks) {
   return nullptr;
 }
 
-void* loss_fn(int precision, uint32_t rp, const void* W, const void* H, bool chunks) {
+void* loss_fn(int precision, uint32_t r, uint32_t rp, const void* W, const void* H, bool zero_pad) {
   if (precision == kFp64) return reinterpret_cast<void*>(&loss_exact_kernel);
-  const LossShape s = loss_shape(precision, rp, W, H);
-  return precision == kFp32 ? loss_fn_of<float>(s, chunks) : loss_fn_of<__nv_bfloat16>(s, chunks);
+  const LossShape s = loss_shape(precision, r, rp, W, H);
+  if (precision == kFp32)
+    return zero_pad ? loss_fn_of<float, false>(s) : loss_fn_of<float, true>(s);
+  return zero_pad ? loss_fn_of<__nv_bfloat16, false>(s) : nullptr;  // only FP32 rows may lack it
 }
 
 // Sum over rows of |X_i - Xold_i| (v[0]) and their maximum (v[1]): groups of
@@ -608,36 +591,18 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partia
 }  // namespace
 
 cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st) {
-  void* fn = loss_fn(precision, a.rp, a.W, a.H, false);
+  void* fn = loss_fn(precision, a.r, a.rp, a.W, a.H, a.zero_pad);
   if (!fn) return cudaErrorInvalidValue;
   LossArgs args = a;
   void* params[] = {&args};
   return cudaLaunchKernel(fn, dim3(grid), dim3(256), params, 0, st);
 }
 
-int loss_ctas_per_sm(int precision, uint32_t rp) {
-  void* fn = loss_fn(precision, rp, nullptr, nullptr, false);
+int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp) {
+  void* fn = loss_fn(precision, r, rp, nullptr, nullptr, true);
   int n = 0;
   if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 256, 0) != cudaSuccess) return 0;
   return n;
-}
-
-cudaError_t launch_nzsl_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
-                               const uint32_t* row, const uint32_t* col, const void* val,
-                               const void* W, const void* H, uint32_t r, uint32_t rp,
-                               double* partials, cudaStream_t st) {
-  if (nchunks == 0) return cudaSuccess;
-  if (precision == kFp64) {
-    nzsl_chunks_exact_kernel<<<nchunks, 256, 0, st>>>(chunks, row, col, (const double*)val,
-                                                      (const double*)W, (const double*)H, r, rp,
-                                                      partials);
-    return cudaGetLastError();
-  }
-  void* fn = loss_fn(precision, rp, W, H, true);
-  if (!fn) return cudaErrorInvalidValue;
-  Entries en{row, col, static_cast<const float*>(val)};
-  void* params[] = {&chunks, &en, &W, &H, &r, &rp, &partials};
-  return cudaLaunchKernel(fn, dim3(nchunks), dim3(256), params, 0, st);
 }
 
 cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
