@@ -14,8 +14,10 @@
 // Adam.  Inputs and results live in pinned host memory that the kernels read
 // and write, so no copy is enqueued.  Measured against one CTA of 64 threads
 // per sample, a row of gradients per sample and copies through the stream:
-// one forward pass of a sample 28.6 -> 17.6 us, gradient of 256 samples 70.4
+// one forward pass of a sample 29.0 -> 19.5 us, gradient of 256 samples 70.4
 // -> 32.8 us (host time of the call).
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace dsgdpp {
@@ -48,7 +50,11 @@ __device__ __forceinline__ float gelu_grad(float x) {
 constexpr int kThreads = 256;
 constexpr int kStride = (kParams + 1 + 3) / 4 * 4;  // a row of partials: gradients, then the loss
 
-__device__ __forceinline__ float quad_sum(float v) {  // over the four threads of a unit
+__device__ __forceinline__ double gelu(double x) {
+  return 0.5 * x * (1.0 + erf(x * 0.70710678118654752));
+}
+template <typename A>
+__device__ __forceinline__ A quad_sum(A v) {  // over the four threads of a unit
   v += __shfl_xor_sync(kFullMask, v, 1);
   return v + __shfl_xor_sync(kFullMask, v, 2);
 }
@@ -56,14 +62,18 @@ __device__ __forceinline__ float quad_sum(float v) {  // over the four threads o
 // Samples [blockIdx.x * per_cta, ...) of the batch, S at a time.  out[b] =
 // clip(net(x_b), -1, 1).  GRAD: this CTA's sums of the gradient of (net(x_b) -
 // y)^2 / batch (unclipped output) and of that loss into row blockIdx.x of
-// partials.  Thread (j, q) works on hidden unit j: on a quarter of its inputs
+// partials.  Outputs, and gradients of few samples, take sums and activations
+// in FP64: one output is one sum of 64 terms that may cancel, and FP32 sums err
+// by 1e-6 of it now and then (FP64 by 5e-8, for 2 us more).  Thread (j, q) works on hidden unit j: on a quarter of its inputs
 // for every sample, then on the unit itself for sample q.
 template <int S, bool GRAD>
 __global__ void __launch_bounds__(kThreads) mlp_kernel(const float* __restrict__ P, const float* X,
                                                        const float* Y, int batch, int per_cta,
                                                        float* out, float* partials) {
+  using A = std::conditional_t<GRAD && S != 1, float, double>;
   const int t = threadIdx.x, j = t >> 2, q = t & 3, warp = t >> 5;
-  __shared__ float xs[S][kIn], h1s[S][kHid], red[kThreads / 32][S];
+  __shared__ float xs[S][kIn];
+  __shared__ A h1s[S][kHid], red[kThreads / 32][S];
   __shared__ float d2s[GRAD ? S : 1][kHid], d1s[GRAD ? S : 1][kHid];
   __shared__ float w2s[GRAD ? kHid : 1][kHid + 1];
   float w1[4], w2[16];
@@ -91,12 +101,12 @@ __global__ void __launch_bounds__(kThreads) mlp_kernel(const float* __restrict__
     const bool mine = q < S && s0 + q < end;  // this thread's sample exists
     const float y = GRAD && mine ? Y[s0 + q] : 0.0f;
     __syncthreads();
-    float z1 = 0, z2 = 0;  // of sample q
+    A z1 = 0, z2 = 0;  // of sample q
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      float a = 0;
+      A a = 0;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) a += w1[c] * xs[s][q * 4 + c];
+      for (int c = 0; c < 4; ++c) a += (A)w1[c] * (A)xs[s][q * 4 + c];
       a = quad_sum(a) + b1;
       if (s == q) z1 = a;
     }
@@ -104,32 +114,33 @@ __global__ void __launch_bounds__(kThreads) mlp_kernel(const float* __restrict__
     __syncthreads();
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      float a = 0;
+      A a = 0;
 #pragma unroll
-      for (int c = 0; c < 16; ++c) a += w2[c] * h1s[s][q * 16 + c];
+      for (int c = 0; c < 16; ++c) a += (A)w2[c] * h1s[s][q * 16 + c];
       a = quad_sum(a) + b2;
       if (s == q) z2 = a;
     }
-    const float h2 = gelu(z2);
-    float o = w3 * h2;  // summed over the units: in the warp, then over the warps
+    const A h2 = gelu(z2);
+    A o = (A)w3 * h2;  // summed over the units: in the warp, then over the warps
 #pragma unroll
     for (int off = 4; off < 32; off <<= 1) o += __shfl_xor_sync(kFullMask, o, off);
     if ((t & 31) < S) red[warp][q] = o;
     __syncthreads();
-    float raw = b3;
+    A raw = b3;
     if (q < S) {
 #pragma unroll
       for (int w = 0; w < kThreads / 32; ++w) raw += red[w][q];
     }
-    if (j == 0 && mine && out) out[s0 + q] = fminf(1.0f, fmaxf(-1.0f, raw));
+    if (j == 0 && mine && out) out[s0 + q] = fminf(1.0f, fmaxf(-1.0f, (float)raw));
     if constexpr (GRAD) {
       // the loss is taken on the unclipped output (the clip applies to the
       // proposed multiplier only), so a saturated output still gets a gradient
-      const float dout = mine ? 2.0f * (raw - y) / (float)batch : 0.0f;
-      if (mine) loss += (raw - y) * (raw - y) / (float)batch;
+      const A miss = raw - (A)y;
+      const float dout = mine ? (float)((A)2 * miss / (A)batch) : 0.0f;
+      if (mine) loss += (float)(miss * miss / (A)batch);
       gb3 += dout;
-      g3 += dout * h2;
-      const float d2 = dout * w3 * gelu_grad(z2);
+      g3 += dout * (float)h2;
+      const float d2 = dout * w3 * gelu_grad((float)z2);
       gb2 += d2;
       if (q < S) d2s[q][j] = d2;
       __syncthreads();
@@ -140,13 +151,13 @@ __global__ void __launch_bounds__(kThreads) mlp_kernel(const float* __restrict__
         float a = 0;
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
-          g2[c] += dj * h1s[s][q * 16 + c];
+          g2[c] += dj * (float)h1s[s][q * 16 + c];
           a += w2s[q * 16 + c][j] * d2s[s][q * 16 + c];
         }
         a = quad_sum(a);
         if (s == q) dh1 = a;
       }
-      const float d1 = dh1 * gelu_grad(z1);
+      const float d1 = dh1 * gelu_grad((float)z1);
       if (q < S) {
         gb1 += d1;
         d1s[q][j] = d1;
