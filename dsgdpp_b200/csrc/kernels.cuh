@@ -177,13 +177,17 @@ int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp);
 cudaError_t launch_sum_partials(const double* partials, uint32_t count, double* out,
                                 cudaStream_t st);
 
-// Per-problem sums of the batched form: one CTA per range chunk writes
-// partials[chunk] (LossArgs::chunks, sumsq_chunks); owner_sums adds partials[owner_begin[p] .. owner_begin[p+1])
-// in order into out[p] for p < owners.
-cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
-                                const void* X, double* partials, cudaStream_t st);
-cudaError_t launch_owner_sums(const double* partials, const uint32_t* owner_begin,
-                              uint32_t owners, double* out, cudaStream_t st);
+// Per-problem sums of the batched form: one CTA per range writes its partial
+// (LossArgs::chunks for squared errors; sumsq_chunks for nw ranges of W, then nh
+// of H); owner_sums adds each owner's partials in order into out[owner.out]
+// (device or pinned host memory).
+cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nw, uint32_t nh,
+                                const void* W, const void* H, double* partials, cudaStream_t st);
+struct OwnerRange {
+  uint32_t begin, end, out;
+};
+cudaError_t launch_owner_sums(const double* partials, const OwnerRange* owners, uint32_t count,
+                              double* out, cudaStream_t st);
 
 // Sum (out[0]) and maximum (out[1]) over the rows of W and of H of their
 // Euclidean move since W0, H0; partials holds 2 * grid doubles, ticket and out

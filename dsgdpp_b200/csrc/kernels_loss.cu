@@ -348,25 +348,28 @@ constexpr int loss_ctas(int N, int V) { return N * V < 16 ? 3 : 2; }
 // ---- per-problem (segmented) reductions of the batched form ----------------------
 // One CTA per chunk of a problem's range; owner_sums then adds each problem's
 // chunk partials in chunk order, so every per-problem sum is deterministic.
+// Sums of squares of ranges of W (the first nw) and of H.
 template <typename T>
-__global__ void __launch_bounds__(256) sumsq_chunks_kernel(const RangeChunk* chunks, const T* X,
+__global__ void __launch_bounds__(256) sumsq_chunks_kernel(const RangeChunk* chunks, uint32_t nw,
+                                                           const T* W, const T* H,
                                                            double* partials) {
   __shared__ double sh[32];
   const RangeChunk c = chunks[blockIdx.x];  // whole rows or pieces of 2^14 elements: whole vectors
-  const double acc = sum_squares<T>(X + c.begin, c.end - c.begin, threadIdx.x, blockDim.x);
+  const double acc = sum_squares<T>((blockIdx.x < nw ? W : H) + c.begin, c.end - c.begin,
+                                    threadIdx.x, blockDim.x);
   const double t = block_reduce(acc, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
+// out[o.out] = the sum of partials [o.begin, o.end), in a fixed order
 __global__ void __launch_bounds__(256) owner_sums_kernel(const double* partials,
-                                                         const uint32_t* owner_begin,
-                                                         double* out) {
+                                                         const OwnerRange* owners, double* out) {
   __shared__ double sh[32];
-  const uint32_t p = blockIdx.x;
+  const OwnerRange o = owners[blockIdx.x];
   double acc = 0;
-  for (uint32_t k = owner_begin[p] + threadIdx.x; k < owner_begin[p + 1]; k += blockDim.x)
+  for (uint32_t k = o.begin + threadIdx.x; k < o.end; k += blockDim.x)
     acc = __dadd_rn(acc, partials[k]);
   const double t = block_reduce(acc, sh);
-  if (threadIdx.x == 0) out[p] = t;
+  if (threadIdx.x == 0) out[o.out] = t;
 }
 
 // ---- one launch per loss --------------------------------------------------------
@@ -605,23 +608,25 @@ int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp) {
   return n;
 }
 
-cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nchunks,
-                                const void* X, double* partials, cudaStream_t st) {
-  if (nchunks == 0) return cudaSuccess;
+cudaError_t launch_sumsq_chunks(int precision, const RangeChunk* chunks, uint32_t nw, uint32_t nh,
+                                const void* W, const void* H, double* partials, cudaStream_t st) {
+  if (nw + nh == 0) return cudaSuccess;
   if (precision == kFp64)
-    sumsq_chunks_kernel<double><<<nchunks, 256, 0, st>>>(chunks, (const double*)X, partials);
+    sumsq_chunks_kernel<double><<<nw + nh, 256, 0, st>>>(chunks, nw, (const double*)W,
+                                                         (const double*)H, partials);
   else if (precision == kFp32)
-    sumsq_chunks_kernel<float><<<nchunks, 256, 0, st>>>(chunks, (const float*)X, partials);
+    sumsq_chunks_kernel<float><<<nw + nh, 256, 0, st>>>(chunks, nw, (const float*)W,
+                                                        (const float*)H, partials);
   else
-    sumsq_chunks_kernel<__nv_bfloat16><<<nchunks, 256, 0, st>>>(
-        chunks, (const __nv_bfloat16*)X, partials);
+    sumsq_chunks_kernel<__nv_bfloat16><<<nw + nh, 256, 0, st>>>(
+        chunks, nw, (const __nv_bfloat16*)W, (const __nv_bfloat16*)H, partials);
   return cudaGetLastError();
 }
 
-cudaError_t launch_owner_sums(const double* partials, const uint32_t* owner_begin,
-                              uint32_t owners, double* out, cudaStream_t st) {
-  if (owners == 0) return cudaSuccess;
-  owner_sums_kernel<<<owners, 256, 0, st>>>(partials, owner_begin, out);
+cudaError_t launch_owner_sums(const double* partials, const OwnerRange* owners, uint32_t count,
+                              double* out, cudaStream_t st) {
+  if (count == 0) return cudaSuccess;
+  owner_sums_kernel<<<count, 256, 0, st>>>(partials, owners, out);
   return cudaGetLastError();
 }
 

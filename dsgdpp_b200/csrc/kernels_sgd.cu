@@ -1071,23 +1071,23 @@ __global__ void __launch_bounds__(256) normalize_kernel(T* W, T* H, uint64_t m, 
   }
 }
 
-template <typename T>
-__global__ void scale_rows_kernel(T* W, uint64_t wrows, T* H, uint64_t hrows, uint32_t rp,
-                                  const uint32_t* w_slot, const uint32_t* h_slot,
-                                  const float* scales) {
-  const uint64_t wtot = wrows * rp, tot = wtot + hrows * rp;
+// The batched form: W row i times scales[w_slot[i]], H row j times
+// scales[h_slot[j]].  16-byte vectors, the row of a vector by a 32-bit division
+// (I) where the sides allow it.
+template <typename T, typename I>
+__global__ void __launch_bounds__(256) scale_rows_kernel(T* W, uint64_t wrows, T* H, uint64_t hrows,
+                                                         uint32_t rp, const uint32_t* w_slot,
+                                                         const uint32_t* h_slot,
+                                                         const float* scales) {
+  const uint32_t vpr = rp / Elem<T>::VW;  // vectors per row
+  const uint64_t wv = wrows * vpr, tot = wv + hrows * vpr;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < tot; q += stride) {
-    if (q < wtot) {
-      const float s = scales[w_slot[q / rp]];
-      if constexpr (sizeof(T) == 8) W[q] *= (double)s;
-      else W[q] = (T)((float)W[q] * s);
-    } else {
-      const uint64_t hq = q - wtot;
-      const float s = scales[h_slot[hq / rp]];
-      if constexpr (sizeof(T) == 8) H[hq] *= (double)s;
-      else H[hq] = (T)((float)H[hq] * s);
-    }
+    const bool in_w = q < wv;
+    const I k = (I)(in_w ? q : q - wv);
+    const float s = scales[(in_w ? w_slot : h_slot)[k / vpr]];
+    uint4* p = reinterpret_cast<uint4*>(in_w ? W : H) + k;
+    *p = scale_vec<T>(*p, s);
   }
 }
 
@@ -1233,18 +1233,30 @@ cudaError_t launch_normalize(int precision, void* W, void* H, uint64_t m, uint64
   return cudaGetLastError();
 }
 
+namespace {
+
+template <typename T>
+void scale_rows(T* W, uint64_t wrows, T* H, uint64_t hrows, uint32_t rp, const uint32_t* w_slot,
+                const uint32_t* h_slot, const float* scales, cudaStream_t st) {
+  if (std::max(wrows, hrows) * (rp / Elem<T>::VW) <= 0xffffffffull)
+    scale_rows_kernel<T, uint32_t><<<1184, 256, 0, st>>>(W, wrows, H, hrows, rp, w_slot, h_slot,
+                                                         scales);
+  else
+    scale_rows_kernel<T, uint64_t><<<1184, 256, 0, st>>>(W, wrows, H, hrows, rp, w_slot, h_slot,
+                                                         scales);
+}
+
+}  // namespace
+
 cudaError_t launch_scale_rows(int precision, void* W, uint64_t wrows, void* H, uint64_t hrows,
                               uint32_t rp, const uint32_t* w_slot, const uint32_t* h_slot,
                               const float* scales, cudaStream_t st) {
   if (precision == kFp64)
-    scale_rows_kernel<double><<<1184, 256, 0, st>>>((double*)W, wrows, (double*)H, hrows, rp,
-                                                    w_slot, h_slot, scales);
+    scale_rows((double*)W, wrows, (double*)H, hrows, rp, w_slot, h_slot, scales, st);
   else if (precision == kFp32)
-    scale_rows_kernel<float><<<1184, 256, 0, st>>>((float*)W, wrows, (float*)H, hrows, rp,
-                                                   w_slot, h_slot, scales);
+    scale_rows((float*)W, wrows, (float*)H, hrows, rp, w_slot, h_slot, scales, st);
   else
-    scale_rows_kernel<__nv_bfloat16><<<1184, 256, 0, st>>>(
-        (__nv_bfloat16*)W, wrows, (__nv_bfloat16*)H, hrows, rp, w_slot, h_slot, scales);
+    scale_rows((__nv_bfloat16*)W, wrows, (__nv_bfloat16*)H, hrows, rp, w_slot, h_slot, scales, st);
   return cudaGetLastError();
 }
 
