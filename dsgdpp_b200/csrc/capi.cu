@@ -187,7 +187,6 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   c->h_params = halloc<EpochParams>(1, "params");
   c->d_params = dalloc<EpochParams>(1, "params");
   c->h_sigma = halloc<float>((size_t)d2 * d * 3, "sigma");
-  c->d_sigma = dalloc<float>((size_t)d2 * d * 3, "sigma");
   c->h_scales = halloc<float>(d2 + 1, "scales");
   c->d_scales = dalloc<float>(d2 + 1, "scales");
   c->d_segs = dalloc<Segment>((size_t)d2 * (d + 1), "segments");
@@ -248,7 +247,7 @@ void destroy_impl(dsgdpp_ctx* c) {
   dfree(c->scratch);
   dfree(c->W_saved); dfree(c->H_saved);
   hfree(c->h_schedule); dfree(c->d_schedule); hfree(c->h_params); dfree(c->d_params);
-  hfree(c->h_sigma); dfree(c->d_sigma); hfree(c->h_scales); dfree(c->d_scales);
+  hfree(c->h_sigma); hfree(c->h_scales); dfree(c->d_scales);
   dfree(c->d_segs); dfree(c->d_counters); dfree(c->d_launches);
   dfree(c->d_done); dfree(c->d_dep_col); hfree(c->h_dep_col); dfree(c->d_ticket);
   hfree(c->h_error);
@@ -592,18 +591,14 @@ void enqueue_hogwild_epoch(dsgdpp_ctx* c, uint32_t s0, uint32_t s1) {
   const bool l2 = lazy_l2(c);
   const bool persistent = c->cfg.launch == DSGDPP_LAUNCH_PERSISTENT;
   if (s0 == 0) {
-  check_cuda(cudaMemcpyAsync(c->d_schedule, c->h_schedule, (size_t)d2 * d * 4,
-                             cudaMemcpyHostToDevice, st), "H2D schedule");
-  check_cuda(cudaMemcpyAsync(c->d_params, c->h_params, sizeof(EpochParams),
-                             cudaMemcpyHostToDevice, st), "H2D params");
-  if (l2) {
-    check_cuda(cudaMemcpyAsync(c->d_sigma, c->h_sigma, (size_t)d2 * d * 3 * 4,
-                               cudaMemcpyHostToDevice, st), "H2D sigma");
-    check_cuda(cudaMemcpyAsync(c->d_scales, c->h_scales, (d2 + 1) * 4, cudaMemcpyHostToDevice,
-                               st), "H2D scales");
-  }
-  SegBuildArgs sb{c->d_params, c->d_schedule, c->mat[0].block_ptr, l2 ? c->d_sigma : nullptr,
-                  c->d_segs, c->d_counters, d, d2};
+  SegBuildArgs sb{};
+  sb.params = c->h_params; sb.schedule = c->h_schedule;
+  sb.sigma = l2 ? c->h_sigma : nullptr;
+  sb.scales = l2 ? c->h_scales : nullptr;
+  sb.block_ptr = c->mat[0].block_ptr;
+  sb.d_params = c->d_params; sb.d_scales = c->d_scales;
+  sb.segs = c->d_segs; sb.counters = c->d_counters;
+  sb.d = d; sb.nb2 = d2;
   check_cuda(launch_build_segments(sb, st), "build_segments");
   if (persistent) {
     check_cuda(cudaMemcpyAsync(c->d_dep_col, c->h_dep_col, (size_t)d2 * d * 4,
@@ -911,16 +906,22 @@ void factor_terms(dsgdpp_ctx* c, int reg, double* w, double* h) {
   if (h) *h = c->h_out[2];
 }
 
-// The configured loss (mf/loss/loss.h:88-112 SumLoss of Nzsl and L2/Nzl2).
-double loss_impl(dsgdpp_ctx* c) {
-  const int reg = c->cfg.loss == DSGDPP_LOSS_NZSL_L2     ? 1
-                  : c->cfg.loss == DSGDPP_LOSS_NZSL_NZL2 ? 2
-                                                         : 0;
-  enqueue_loss(c, DSGDPP_TRAIN, reg, c->h_out);
-  check_cuda(cudaStreamSynchronize(c->stream), "sync");
+// The configured loss (mf/loss/loss.h:88-112 SumLoss of Nzsl and L2/Nzl2): the
+// factor terms it needs, and its value once h_out[0 .. 2] hold them.
+int loss_reg(const dsgdpp_ctx* c) {
+  return c->cfg.loss == DSGDPP_LOSS_NZSL_L2 ? 1 : c->cfg.loss == DSGDPP_LOSS_NZSL_NZL2 ? 2 : 0;
+}
+
+double loss_value(const dsgdpp_ctx* c) {
   double l = c->h_out[0];
-  if (reg) l = l + c->cfg.loss_lambda * (c->h_out[1] + c->h_out[2]);
+  if (loss_reg(c)) l = l + c->cfg.loss_lambda * (c->h_out[1] + c->h_out[2]);
   return l;
+}
+
+double loss_impl(dsgdpp_ctx* c) {
+  enqueue_loss(c, DSGDPP_TRAIN, loss_reg(c), c->h_out);
+  check_cuda(cudaStreamSynchronize(c->stream), "sync");
+  return loss_value(c);
 }
 
 double elapsed_ns(std::chrono::steady_clock::time_point a, std::chrono::steady_clock::time_point b) {
@@ -1380,6 +1381,20 @@ int dsgdpp_run(dsgdpp_ctx* c, uint32_t epochs, int decay, double eps0, double de
     double prev = 0, eps_state = eps0;
     const uint32_t d = c->d;
     std::vector<uint32_t> sched((size_t)c->nb2 * d), seeds(d);
+    struct Events {  // the end of an epoch's launches, of its loss, of its test loss
+      cudaEvent_t e[3] = {};
+      ~Events() {
+        for (cudaEvent_t v : e)
+          if (v) cudaEventDestroy(v);
+      }
+    } ev;
+    for (cudaEvent_t& v : ev.e) check_cuda(cudaEventCreate(&v), "event");
+    auto between_ns = [&](int from, int to) {
+      float ms = 0;
+      check_cuda(cudaEventElapsedTime(&ms, ev.e[from], ev.e[to]), "elapsed");
+      return (double)ms * 1e6;
+    };
+    if (epochs) draw_epoch(c, sched.data(), seeds.data());
     for (uint32_t e = 0; e < epochs; ++e) {
       auto a = clock::now();
       double eps;
@@ -1392,18 +1407,27 @@ int dsgdpp_run(dsgdpp_ctx* c, uint32_t epochs, int decay, double eps0, double de
         eps = eps_state;
       }
       auto b = clock::now();
-      draw_epoch(c, sched.data(), seeds.data());
+      // the epoch and its losses follow one another on the stream and are
+      // waited for once; the next epoch's draws (which depend on nothing the
+      // epoch computes) are made meanwhile
       epoch_explicit_impl(c, eps, sched.data(), seeds.data());
-      check_cuda(cudaEventSynchronize(c->ev_end), "event sync");
-      auto e1 = clock::now();
+      check_cuda(cudaEventRecord(ev.e[0], c->stream), "event");
+      enqueue_loss(c, DSGDPP_TRAIN, loss_reg(c), c->h_out);
+      check_cuda(cudaEventRecord(ev.e[1], c->stream), "event");
+      if (has_test) enqueue_loss(c, DSGDPP_TEST, 0, c->h_out + 3);
+      check_cuda(cudaEventRecord(ev.e[2], c->stream), "event");
+      if (e + 1 < epochs) draw_epoch(c, sched.data(), seeds.data());
+      check_cuda(cudaEventSynchronize(ev.e[2]), "event sync");
+      auto end = clock::now();
       prev = cur;
-      cur = loss_impl(c);
-      auto e2 = clock::now();
-      test = has_test ? nzsl_impl(c, DSGDPP_TEST) : NAN;
-      auto e3 = clock::now();
-      if (trace)
-        trace[e + 1] = dsgdpp_trace_row{e + 1u, cur, test, eps, elapsed_ns(a, b), elapsed_ns(b, e1),
-                                        elapsed_ns(e1, e2), has_test ? elapsed_ns(e2, e3) : 0.0};
+      cur = loss_value(c);
+      test = has_test ? c->h_out[3] : NAN;
+      if (trace) {
+        const double loss_ns = between_ns(0, 1), test_ns = has_test ? between_ns(1, 2) : 0.0;
+        trace[e + 1] = dsgdpp_trace_row{e + 1u, cur, test, eps, elapsed_ns(a, b),
+                                        std::max(0.0, elapsed_ns(b, end) - loss_ns - test_ns),
+                                        loss_ns, test_ns};
+      }
     }
     return DSGDPP_OK;
   });

@@ -95,13 +95,12 @@ struct dsgdpp_ctx {
   size_t scratch_bytes = 0;
   void* W_saved = nullptr;    // factor snapshot (dsgdpp_save_factors)
   void* H_saved = nullptr;
-  // per-epoch inputs (pinned host copies feed the device copies)
+  // per-epoch inputs (pinned; a Hogwild epoch reads them there, the replay copies them)
   uint32_t* h_schedule = nullptr;
   uint32_t* d_schedule = nullptr;
   EpochParams* h_params = nullptr;
   EpochParams* d_params = nullptr;
   float* h_sigma = nullptr;   // [2d][d][3]
-  float* d_sigma = nullptr;
   float* h_scales = nullptr;  // [2d + 1]
   float* d_scales = nullptr;
   Segment* d_segs = nullptr;

@@ -67,10 +67,14 @@ struct ReplayArgs {
 };
 
 struct SegBuildArgs {
-  const EpochParams* params;  // eps of the epoch
+  // page-locked host memory, read by the launch
+  const EpochParams* params;  // of the epoch
   const uint32_t* schedule;   // [nb2][d]
-  const uint64_t* block_ptr;  // d*nb2+1
   const float* sigma;         // [nb2][d][3] lazy L2 scales, or null (all ones)
+  const float* scales;        // [nb2 + 1] for the end of the epoch, or null
+  const uint64_t* block_ptr;  // d*nb2+1
+  EpochParams* d_params;      // the launch's copies of params and scales
+  float* d_scales;
   Segment* segs;              // [nb2][d+1]
   uint32_t* counters;         // [nb2]
   uint32_t d;
