@@ -339,7 +339,9 @@ int dsgdpp_nzsl_fp32_noalloc(const uint32_t* rows, const uint32_t* cols, const f
 /* replaces: DsgdPpRunner::run -> detail::defaultRunner (mf/sgd/sgd_impl.h:34-145):
  * loss and test loss, then per epoch: decay, epoch, loss, test loss.  trace
  * receives epochs+1 rows (row 0 = the initial losses, eps NaN).  The test loss
- * is skipped (NaN) when no test matrix was set. */
+ * is skipped (NaN) when no test matrix was set.  An epoch and its losses are
+ * waited for together: from row 1 on time_loss and time_test_loss are their
+ * times on the device, time_epoch the rest of the wall time. */
 int dsgdpp_run(dsgdpp_ctx* ctx, uint32_t epochs, int decay, double eps0, double decrease,
                double increase, dsgdpp_trace_row* trace);
 int dsgdpp_sync(dsgdpp_ctx* ctx);
