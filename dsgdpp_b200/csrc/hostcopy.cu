@@ -5,7 +5,6 @@
 #include <cstring>
 #include <mutex>
 #include <system_error>
-#include <vector>
 
 namespace dsgdpp {
 namespace {
@@ -24,47 +23,46 @@ constexpr size_t kMaxSlabs = 2;  // 32 MB
 constexpr size_t kSlabAfter = 64 << 20;
 
 std::mutex g_mutex;
-std::vector<void*> g_slabs;
-std::vector<void*> g_free;  // pieces not in use
+void* g_slabs[kMaxSlabs];
+size_t g_nslabs = 0;
+void* g_free[kMaxSlabs * kSlabPieces];  // pieces not in use
+size_t g_nfree = 0;
 size_t g_holders = 0;
-size_t g_copied = 0;        // bytes copied directly since there was no slab
+size_t g_copied = 0;  // bytes copied directly since there was no slab
 
 void free_slabs_if_unused() {  // under the mutex
-  if (g_slabs.empty() || g_holders > 0 || g_free.size() != g_slabs.size() * kSlabPieces) return;
-  for (void* p : g_slabs) cudaFreeHost(p);
-  g_slabs.clear();
-  g_free.clear();
+  if (g_nslabs == 0 || g_holders > 0 || g_nfree != g_nslabs * kSlabPieces) return;
+  for (size_t k = 0; k < g_nslabs; ++k) cudaFreeHost(g_slabs[k]);
+  g_nslabs = g_nfree = 0;
   g_copied = 0;
 }
 
 bool worth_staging(size_t bytes) {
   std::lock_guard<std::mutex> lock(g_mutex);
-  if (!g_slabs.empty()) return true;
+  if (g_nslabs > 0) return true;
   g_copied += bytes;
   return g_copied >= kSlabAfter;
 }
 
 void* take_piece() {
   std::lock_guard<std::mutex> lock(g_mutex);
-  if (g_free.empty()) {
-    if (g_slabs.size() >= kMaxSlabs) return nullptr;
+  if (g_nfree == 0) {
+    if (g_nslabs >= kMaxSlabs) return nullptr;
     void* p = nullptr;
     if (cudaHostAlloc(&p, kPiece * kSlabPieces, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();  // not an error of the copy: it goes the direct way
       return nullptr;
     }
-    g_slabs.push_back(p);
-    for (size_t k = kSlabPieces; k-- > 0;) g_free.push_back(static_cast<char*>(p) + k * kPiece);
+    g_slabs[g_nslabs++] = p;
+    for (size_t k = 0; k < kSlabPieces; ++k) g_free[g_nfree++] = static_cast<char*>(p) + k * kPiece;
   }
-  void* p = g_free.back();
-  g_free.pop_back();
-  return p;
+  return g_free[--g_nfree];
 }
 
 void give_piece(void* p) {
   if (!p) return;
   std::lock_guard<std::mutex> lock(g_mutex);
-  g_free.push_back(p);
+  g_free[g_nfree++] = p;
   free_slabs_if_unused();
 }
 
