@@ -302,6 +302,11 @@ __device__ __forceinline__ double sum_squares(const T* X, uint64_t count, uint64
 
 // Lanes that share a row of `vpr` 16-byte vectors in the row-wise sums: the
 // power of two that covers it (at most 32), so rows are read coalesced.
+// The row-wise sums below read with the default cache policy: they run between
+// epochs, and evict-first loads would take the factors out of L2 that the next
+// epoch starts on -- which is how stale its first reads are, and moved the loss
+// trace (3M entries, rank 50, ten epochs with this loss after each: by 1.4
+// times what one run differs by from another).
 __device__ __forceinline__ uint32_t row_lanes(uint32_t vpr) {
   uint32_t l = 1;
   while (l < vpr && l < 32) l <<= 1;
@@ -328,7 +333,7 @@ __device__ __forceinline__ double weighted_squares(const T* X, uint64_t rows, ui
         x[u] = make_uint4(0, 0, 0, 0);
         c[u] = 0;
         if (i < rows) {
-          x[u] = __ldcs(V + i * vpr + v);
+          x[u] = V[i * vpr + v];
           c[u] = (double)cnt[i];
         }
       }
@@ -542,8 +547,8 @@ __device__ __forceinline__ void row_moves(const T* X, const T* Xold, uint64_t ro
         const uint64_t i = k0 + u * groups + tid / lanes;
         x[u] = y[u] = make_uint4(0, 0, 0, 0);
         if (i < rows) {
-          x[u] = __ldcs(A + i * vpr + v);
-          y[u] = __ldcs(B + i * vpr + v);
+          x[u] = A[i * vpr + v];
+          y[u] = B[i * vpr + v];
         }
       }
 #pragma unroll

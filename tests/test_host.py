@@ -153,3 +153,15 @@ def test_mlp_oracle_gradient_matches_finite_differences():
         e[k] = 1e-6
         num = (M.loss_and_grad(p + e, X, y)[0] - M.loss_and_grad(p - e, X, y)[0]) / 2e-6
         assert g[k] == pytest.approx(num, rel=1e-5, abs=1e-9)
+
+
+@pytest.mark.parametrize("function", ["weighted_squares", "row_moves"])
+def test_row_sums_between_epochs_leave_the_factors_cached(function):
+    # evict-first loads here change what the next epoch finds in L2, and with
+    # it when its updates see each other
+    with open(os.path.join(ROOT, "dsgdpp_b200", "csrc", "kernels_loss.cu")) as f:
+        text = f.read()
+    body = text[re.search(r"__device__ __forceinline__ \w+ %s\(" % function, text).start():]
+    body = body[:body.index("\n}\n")]
+    assert "row_lanes(" in body
+    assert not re.search(r"__ldcs|__ldlu|evict|no_allocate", body)
