@@ -556,7 +556,6 @@ void losses(dsgdpp_batch* b, bool test) {
     a.row = G.row; a.col = G.col; a.val = G.val;
     a.W = G.W; a.H = G.H;
     a.r = a.rp = G.rp;
-    a.zero_pad = true;
     a.partials = b->d_partials + G.n0;
     a.chunks = G.d_nchunks;
     if (G.nn) check_cuda(launch_loss(prec, a, G.nn, st), "loss");

@@ -881,7 +881,6 @@ void enqueue_loss(dsgdpp_ctx* c, int which, int reg, double* out) {
   a.W = c->W; a.H = c->H;
   a.m = c->cfg.m; a.n = c->cfg.n;
   a.r = c->r; a.rp = c->rp;
-  a.zero_pad = true;
   a.reg = reg;
   a.cnt1 = c->cnt1; a.cnt2 = c->cnt2;
   a.partials = c->d_partials;

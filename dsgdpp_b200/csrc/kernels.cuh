@@ -164,8 +164,7 @@ struct LossArgs {
   const void* W;
   const void* H;
   uint64_t m, n;
-  uint32_t r, rp;
-  bool zero_pad;         // rows hold zeros from r to rp (may be false for FP32)
+  uint32_t r, rp;  // without `reg` a row may hold anything from r to rp
   int reg;
   const uint32_t* cnt1;  // reg 2: nnz1, nnz2
   const uint32_t* cnt2;

@@ -108,8 +108,10 @@ constexpr int kLossWords = 16;
 
 // The squared error of 32 entries (nrec of them exist; the others name rows
 // that exist), one entry per lane in the end.  A lane whose vector starts past
-// the rank reads the row's first one and drops it; with MASK a vector that
-// reaches past the rank is masked there (rows whose padding is not zero).
+// the rank reads the row's first one and drops it; with MASK (the rank is no
+// whole number of vectors) a vector that reaches past the rank is masked there:
+// a caller's padding may hold anything, and a context's holds NaN once an
+// update was infinite.
 template <typename T, int L, int V, int N, bool MASK>
 __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, float my_val,
                                             uint32_t nrec, const T* W, const T* H, uint32_t r,
@@ -524,12 +526,12 @@ void* loss_fn_of(LossShape s) {
   return nullptr;
 }
 
-void* loss_fn(int precision, uint32_t r, uint32_t rp, const void* W, const void* H, bool zero_pad) {
+void* loss_fn(int precision, uint32_t r, uint32_t rp, const void* W, const void* H) {
   if (precision == kFp64) return reinterpret_cast<void*>(&loss_exact_kernel);
   const LossShape s = loss_shape(precision, r, rp, W, H);
-  if (precision == kFp32)
-    return zero_pad ? loss_fn_of<float, false>(s) : loss_fn_of<float, true>(s);
-  return zero_pad ? loss_fn_of<__nv_bfloat16, false>(s) : nullptr;  // only FP32 rows may lack it
+  const bool mask = r * (precision == kFp32 ? 4u : 2u) % (4u * s.words) != 0;
+  if (precision == kFp32) return mask ? loss_fn_of<float, true>(s) : loss_fn_of<float, false>(s);
+  return mask ? loss_fn_of<__nv_bfloat16, true>(s) : loss_fn_of<__nv_bfloat16, false>(s);
 }
 
 // Sum over rows of |X_i - Xold_i| (v[0]) and their maximum (v[1]): groups of
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partia
 }  // namespace
 
 cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st) {
-  void* fn = loss_fn(precision, a.r, a.rp, a.W, a.H, a.zero_pad);
+  void* fn = loss_fn(precision, a.r, a.rp, a.W, a.H);
   if (!fn) return cudaErrorInvalidValue;
   LossArgs args = a;
   void* params[] = {&args};
@@ -613,7 +615,7 @@ cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStr
 }
 
 int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp) {
-  void* fn = loss_fn(precision, r, rp, nullptr, nullptr, true);
+  void* fn = loss_fn(precision, r, rp, nullptr, nullptr);
   int n = 0;
   if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 256, 0) != cudaSuccess) return 0;
   return n;

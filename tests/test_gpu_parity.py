@@ -758,3 +758,20 @@ def test_matrix_from_pageable_and_page_locked_arrays(nnz):
                 ctx.set_matrix(P.TRAIN, give(bad), give(cols), give(vals))
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("r", [3, 10, 50, 130])
+def test_losses_of_infinite_factors_leave_out_the_rows_padding(r):
+    # an infinite step times the padding's zeros is NaN; the loss of the
+    # factors themselves is infinite
+    with P.Context(P.Config(m=4, n=4, rank=r, d=1, precision="fp32", update="Nzsl", loss="Nzsl",
+                            lanes_per_nnz=32 if r > 128 else 0)) as ctx:
+        at = np.zeros(1, np.uint32)
+        ctx.set_matrix(P.TRAIN, at, at, np.ones(1))
+        ctx.set_matrix(P.TEST, at, at, np.ones(1))
+        ctx.set_factors(np.full((4, r), 1e20), np.full((4, r), 1e20))
+        ctx.seed(1)
+        ctx.epoch(0.01)
+        W, H = ctx.get_factors()
+        assert (1.0 - W[0] @ H[0]) ** 2 == np.inf
+        assert ctx.loss() == np.inf and ctx.nzsl(P.TEST) == np.inf
