@@ -159,8 +159,10 @@ def test_mlp_oracle_gradient_matches_finite_differences():
 def test_row_sums_between_epochs_leave_the_factors_cached(function):
     # evict-first loads here change what the next epoch finds in L2, and with
     # it when its updates see each other
-    with open(os.path.join(ROOT, "dsgdpp_b200", "csrc", "kernels_loss.cu")) as f:
-        text = f.read()
+    text = ""
+    for name in ("loss_rows.cuh", "kernels_loss.cu"):
+        with open(os.path.join(ROOT, "dsgdpp_b200", "csrc", name)) as f:
+            text += f.read()
     body = text[re.search(r"__device__ __forceinline__ \w+ %s\(" % function, text).start():]
     body = body[:body.index("\n}\n")]
     assert "row_lanes(" in body
