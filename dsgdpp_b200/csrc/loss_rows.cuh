@@ -117,7 +117,8 @@ __device__ __forceinline__ uint32_t elem_bits(const Words<N>& v, int e) {
 constexpr int kLossWords = 16;
 
 // The squared error of 32 entries (nrec of them exist; the others name rows
-// that exist), one entry per lane in the end.  A lane whose vector starts past
+// that an entry names: no other row of W or H need be memory of the caller's),
+// one entry per lane in the end.  A lane whose vector starts past
 // the rank reads the row's first one and drops it; with MASK (the rank is no
 // whole number of vectors) a vector that reaches past the rank is masked there:
 // a caller's padding may hold anything, and a context's holds NaN once an
@@ -219,12 +220,13 @@ __device__ __forceinline__ double nzsl_lanes(const LossArgs& a, uint64_t begin, 
   const float* val = static_cast<const float*>(a.val);
   double acc = 0;
   uint64_t base = begin + warp * 32;
-  uint32_t n_row = 0, n_col = 0;  // of a lane without an entry: row 0, or an earlier entry's
+  uint32_t n_row = 0, n_col = 0;  // of a lane without an entry: those of an earlier one
   float n_val = 0;
-  if (base + lane < end) {
-    n_row = a.row[base + lane];
-    n_col = a.col[base + lane];
-    n_val = val[base + lane];
+  if (base < end) {
+    const uint64_t k = min(base + lane, end - 1);
+    n_row = a.row[k];
+    n_col = a.col[k];
+    n_val = val[k];
   }
   for (; base < end; base += nwarps * 32) {
     const uint32_t my_row = n_row, my_col = n_col;

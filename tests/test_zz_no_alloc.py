@@ -107,3 +107,26 @@ def test_noalloc_leaves_padding_and_alignment_to_the_caller(r, ld, shift):
     f = lambda a: a.astype(np.float32).astype(np.float64)
     want = np.sum((f(p.vals) - np.einsum("ij,ij->i", f(p.W0)[p.rows], f(p.H0)[p.cols])) ** 2)
     assert got == pytest.approx(float(want), rel=LOSS_RTOL)
+
+
+@pytest.mark.parametrize("nnz", [1, 31, 33, 2000])
+def test_noalloc_reads_only_the_rows_that_entries_name(nnz):
+    # the bases point 1000 rows before the callers' memory, as those of a part
+    # of a larger matrix do
+    import torch
+    r, ld, first = 30, 32, 1000
+    p = synth.make(300, 200, 4000, 10, rank_true=5, r=r, noise=0.1, seed=nnz)
+    W, H = _padded(torch, p.W0, ld), _padded(torch, p.H0, ld)
+    rows, cols, vals = p.rows[:nnz], p.cols[:nnz], p.vals[:nnz]
+    out = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+    dr = _device(torch, (rows + np.uint32(first)).view(np.int32), torch.int32)
+    dc = _device(torch, (cols + np.uint32(first)).view(np.int32), torch.int32)
+    dv = _device(torch, vals, torch.float32)
+    back = first * ld * 4
+    assert P.lib.dsgdpp_nzsl_fp32_noalloc(
+        dr.data_ptr(), dc.data_ptr(), dv.data_ptr(), nnz, W.data_ptr() - back,
+        H.data_ptr() - back, r, ld, 0, out.data_ptr(), None) == P.OK
+    torch.cuda.synchronize()
+    f = lambda a: a.astype(np.float32).astype(np.float64)
+    want = np.sum((f(vals) - np.einsum("ij,ij->i", f(p.W0)[rows], f(p.H0)[cols])) ** 2)
+    assert float(out.item()) == pytest.approx(float(want), rel=LOSS_RTOL)
