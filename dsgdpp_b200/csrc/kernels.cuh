@@ -174,6 +174,9 @@ struct LossArgs {
   double* out;
 };
 cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st);
+// Loads the modules of the FP32 loss kernels into the current context, so that
+// no later launch does.
+cudaError_t load_fp32_loss_kernels();
 // CTAs per SM of the loss kernel for this precision, rank and row width
 int loss_ctas_per_sm(int precision, uint32_t r, uint32_t rp);
 // out[0] = the sum of `count` partials

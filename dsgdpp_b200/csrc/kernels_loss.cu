@@ -178,6 +178,13 @@ __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partia
 
 }  // namespace
 
+cudaError_t load_fp32_loss_kernels() {
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, loss_kernel_fp32(LossShape{1, 1, 8}, false));
+  if (e != cudaSuccess) return e;
+  return cudaFuncGetAttributes(&at, loss_kernel_fp32_long(LossShape{8, 4, 8}, false));
+}
+
 cudaError_t launch_loss(int precision, const LossArgs& a, uint32_t grid, cudaStream_t st) {
   void* fn = loss_fn(precision, a.r, a.rp, a.W, a.H);
   if (!fn) return cudaErrorInvalidValue;

@@ -58,7 +58,8 @@ cudaError_t current_context(CUcontext* ctx) {
 }
 
 // Once per context, with its device current: the device address of the
-// scratch array and the SM count.
+// scratch array, the SM count, and the kernels' modules (later calls may be
+// captured and allocate nothing).
 cudaError_t context_setup(int dev, double** scratch, int* sms) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   // a runtime call first, so the device's primary context exists and is current
@@ -77,6 +78,7 @@ cudaError_t context_setup(int dev, double** scratch, int* sms) {
   if (g_nsetup == kMaxContexts) return cudaErrorDeviceUninitialized;
   void* p = nullptr;
   e = cudaGetSymbolAddress(&p, g_noalloc_partials);
+  if (e == cudaSuccess) e = dsgdpp::load_fp32_loss_kernels();
   if (e != cudaSuccess) return e;
   g_setup[g_nsetup++] = Setup{ctx, static_cast<double*>(p), n};
   *scratch = static_cast<double*>(p);

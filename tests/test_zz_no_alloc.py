@@ -130,3 +130,24 @@ def test_noalloc_reads_only_the_rows_that_entries_name(nnz):
     f = lambda a: a.astype(np.float32).astype(np.float64)
     want = np.sum((f(vals) - np.einsum("ij,ij->i", f(p.W0)[rows], f(p.H0)[cols])) ** 2)
     assert float(out.item()) == pytest.approx(float(want), rel=LOSS_RTOL)
+
+
+def test_noalloc_calls_of_any_rank_are_captured_after_the_first_call():
+    import torch
+    p = synth.make(300, 200, 2000, 10, rank_true=5, r=200, noise=0.1, seed=3)
+    ids = [_device(torch, a.view(np.int32), torch.int32) for a in (p.rows, p.cols)]
+    v = _device(torch, p.vals, torch.float32)
+    W, H = _padded(torch, p.W0, 200), _padded(torch, p.H0, 200)
+    want = [_call(torch, *ids, v, W, H, 20, 200)]
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        st = torch.cuda.current_stream().cuda_stream
+        for k, r in enumerate((20, 200)):  # the two lengths of rows
+            assert P.lib.dsgdpp_nzsl_fp32_noalloc(
+                *[a.data_ptr() for a in (*ids, v)], v.numel(), W.data_ptr(), H.data_ptr(), r, 200,
+                0, out[k:].data_ptr(), st) == P.OK
+    graph.replay()
+    torch.cuda.synchronize()
+    want.append(_call(torch, *ids, v, W, H, 200, 200))
+    assert out.tolist() == want
