@@ -297,7 +297,9 @@ int dsgdpp_launch_shape(dsgdpp_ctx* ctx, uint32_t* lanes, uint32_t* vecs, uint32
 /* replaces: the configured training loss, SumLoss<NzslLoss, L2Loss|Nzl2Loss>
  * or NzslLoss (mf/loss/loss.h:88-112) */
 int dsgdpp_loss(dsgdpp_ctx* ctx, double* out);
-/* replaces: NzslLoss (mf/loss/nzsl.h:160-185); which = TRAIN or TEST */
+/* replaces: NzslLoss (mf/loss/nzsl.h:160-185); which = TRAIN or TEST.  With FP32
+ * or BF16 factors an element of H that is not finite counts as a number of
+ * 2^128 to 2^129 (one of W as what it is); dsgdpp_l2 sees both. */
 int dsgdpp_nzsl(dsgdpp_ctx* ctx, int which, double* out);
 /* replaces: l2 over W and over H (mf/loss/l2.h:134-145) */
 int dsgdpp_l2(dsgdpp_ctx* ctx, double* w2, double* h2);
