@@ -308,8 +308,10 @@ __device__ __forceinline__ uint32_t row_lanes(uint32_t vpr) {
   return l;
 }
 
-// sum_i cnt[i] |X_i|^2 (Nzl2Loss, mf/loss/nzl2.h) over rows dealt to groups of
-// lanes; each lane weighs its own share of a row, four rows in flight.
+// sum_i cnt[i] |X_i|^2 (Nzl2Loss, mf/loss/nzl2.h).  FP64 rows are summed by a
+// thread each, in z order, and then weighed, as the reference does.  FP32 and
+// BF16 rows are dealt to groups of lanes; each lane weighs its own share of a
+// row, four rows in flight.
 template <typename T>
 __device__ __forceinline__ double weighted_squares(const T* X, uint64_t rows, uint32_t rp,
                                                    const uint32_t* cnt, uint64_t tid,
@@ -318,6 +320,15 @@ __device__ __forceinline__ double weighted_squares(const T* X, uint64_t rows, ui
   const uint4* V = reinterpret_cast<const uint4*>(X);
   const uint64_t groups = stride / lanes;
   double acc = 0;
+  if constexpr (sizeof(T) == 8) {
+    for (uint64_t i = tid; i < rows; i += stride) {
+      double row = 0;
+#pragma unroll 4
+      for (uint32_t v = 0; v < vpr; ++v) row = add_squares<T>(row, V[i * vpr + v]);
+      acc = __dadd_rn(acc, __dmul_rn((double)cnt[i], row));
+    }
+    return acc;
+  }
   for (uint64_t i0 = tid / lanes; i0 < rows; i0 += 4 * groups) {
     for (uint32_t v = gl; v < vpr; v += lanes) {
       uint4 x[4];

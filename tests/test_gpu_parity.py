@@ -775,3 +775,25 @@ def test_losses_of_infinite_factors_leave_out_the_rows_padding(r):
         W, H = ctx.get_factors()
         assert (1.0 - W[0] @ H[0]) ** 2 == np.inf
         assert ctx.loss() == np.inf and ctx.nzsl(P.TEST) == np.inf
+
+
+@pytest.mark.parametrize("r", [2, 7, 10, 33, 64, 255])
+def test_fp64_nonzero_weighted_loss_forms_each_row_as_the_reference(r):
+    # one row of each factor is not zero, so the sum over the rows is exact
+    rng = np.random.default_rng(r)
+    m, n = 50, 40
+    keys = rng.permutation(m * n)[:900]
+    rows, cols = (keys // n).astype(np.uint32), (keys % n).astype(np.uint32)
+    with P.Context(P.Config(m=m, n=n, rank=r, d=2, precision="fp64")) as ctx:
+        ctx.set_matrix(P.TRAIN, rows, cols, rng.standard_normal(900))
+        for i, j in ((0, 0), (17, 23), (m - 1, n - 1)):
+            W, H = np.zeros((m, r)), np.zeros((n, r))
+            W[i], H[j] = rng.standard_normal(r), rng.standard_normal(r)
+            ctx.set_factors(W, H)
+            want = []
+            for x, count in ((W[i], np.sum(rows == i)), (H[j], np.sum(cols == j))):
+                total = 0.0
+                for z in range(r):
+                    total += float(x[z]) * float(x[z])
+                want.append(float(count) * total)
+            assert ctx.nzl2() == tuple(want)
