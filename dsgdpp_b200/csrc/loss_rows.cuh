@@ -119,6 +119,14 @@ __device__ __forceinline__ uint32_t elem_bits(const Words<N>& v, int e) {
 // vector words of each side that a lane has in flight (8: 0.27 against 0.26 ms
 // at BF16 rank 32; 32 spill, or halve the warps)
 constexpr int kLossWords = 16;
+// BF16 rows of 32 lanes with four vectors (ranks from 769 that fill no 32-byte
+// vector) take 8, and test for a ragged rank at run time: the sums of 32 lanes
+// leave no registers for more, and the test keeps the unpacking of a row's last
+// vector behind that of the others.  2M entries, 16 words / 8 / 8 and the test:
+// rank 776 1063 / - / 971 us, 1000 1110 / 1144 / 975 (16-byte loads, a
+// butterfly per round: 997).  FP32 is slower so (rank 508: 473 -> 709).
+template <typename T, int L, int V>
+constexpr bool kTight = sizeof(T) == 2 && L == 32 && V == 4;
 
 // The squared error of 32 entries (nrec of them exist; the others name rows
 // that an entry names: no other row of W or H need be memory of the caller's),
@@ -135,7 +143,7 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
   constexpr int EPV = N * 4 / (int)sizeof(T);  // elements per vector
   // vectors of each side that a lane has in flight: U rounds of a row's V, or
   // C of one round's
-  constexpr int F = kLossWords / N;
+  constexpr int F = (kTight<T, L, V> ? 8 : kLossWords) / N;
   constexpr int C = V < F ? V : F;
   constexpr int U = F / V < 1 ? 1 : F / V < L ? F / V : L;
   const uint32_t lane = threadIdx.x & 31u, grp = lane / L, gl = lane % L;
@@ -171,7 +179,7 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (v0 + c >= V) continue;
-          if (MASK && v0 + c == V - 1) {
+          if ((kTight<T, L, V> ? r % EPV != 0 : MASK) && v0 + c == V - 1) {
 #pragma unroll
             for (int k = 0; k < N; ++k) {
               // whole words past the rank, and the upper half of one that ends it
