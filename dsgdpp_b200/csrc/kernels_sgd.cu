@@ -392,7 +392,12 @@ __global__ void __launch_bounds__(HogwildLaunch<T, LPN, VPL>::threads,
     seg = ss;
   }
   const uint32_t total = seg[nseg].chunk_begin;
-  if (total == 0 || nseg == 0) return;
+  if (total == 0 || nseg == 0) {
+    // nothing to do, but the grid after this one takes this one's end for the
+    // end of all before it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const uint32_t warps = blockDim.x >> 5;
   const uint32_t stride = gridDim.x * warps;  // warps in the grid
   uint32_t lc = blockIdx.x * warps + (threadIdx.x >> 5);
