@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 
 namespace dsgdpp {
 namespace {
@@ -156,7 +155,7 @@ cudaError_t copy(void* dst, const void* src, size_t bytes, bool to_host, int dev
   for (; started < n; ++started) {
     try {
       pool[started] = std::thread(one, started);
-    } catch (const std::system_error&) {
+    } catch (...) {  // std::system_error, std::bad_alloc
       break;  // no more threads: this one does the rest
     }
   }
@@ -190,7 +189,7 @@ void BackgroundCopy::start(void* dst, const void* src, size_t bytes, int device,
   }
   try {
     thread_ = std::thread(run);
-  } catch (const std::system_error&) {
+  } catch (...) {
     run();
   }
 }
