@@ -2,6 +2,8 @@
 #include "hostcopy.h"
 
 #include <algorithm>
+#include <atomic>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 
@@ -15,8 +17,9 @@ constexpr size_t kPiece = 1 << 20;
 constexpr size_t kDirect = 2 << 20;  // below this the driver's own path is as fast
 constexpr unsigned kThreads = 8;
 // One slab serves one copy.  Page-locking it costs some 7 ms, what the pieces
-// save on about 90 MB, so the first is made once that much has been copied
-// (a program that loads little never pays for it).
+// save on about 90 MB, so the first is made once some of that order has been
+// copied: until then, and again after the last holder is gone, copies go the
+// direct way (a program that loads little never pays for the slab).
 constexpr size_t kSlabPieces = 2 * kThreads;
 constexpr size_t kMaxSlabs = 2;  // 32 MB
 constexpr size_t kSlabAfter = 64 << 20;
@@ -28,6 +31,7 @@ void* g_free[kMaxSlabs * kSlabPieces];  // pieces not in use
 size_t g_nfree = 0;
 size_t g_holders = 0;
 size_t g_copied = 0;  // bytes copied directly since there was no slab
+std::atomic<uint64_t> g_staged{0};  // bytes that went through pieces (dsgdpp_staged_bytes)
 
 void free_slabs_if_unused() {  // under the mutex
   if (g_nslabs == 0 || g_holders > 0 || g_nfree != g_nslabs * kSlabPieces) return;
@@ -120,6 +124,7 @@ cudaError_t work(char* dst, const char* src, size_t bytes, size_t first, size_t 
     s.at = at;
     s.len = len;
     s.busy = e == cudaSuccess;
+    if (s.busy) g_staged += len;
   }
   for (int j = 0; j < 2; ++j) {  // in the order they were started
     const cudaError_t r = finish(slot[k ^ j]);
@@ -211,3 +216,5 @@ void hostcopy_drop() {
 }
 
 }  // namespace dsgdpp
+
+extern "C" uint64_t dsgdpp_staged_bytes() { return dsgdpp::g_staged; }

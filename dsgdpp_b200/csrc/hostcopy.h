@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 #include <thread>
 
 namespace dsgdpp {
@@ -43,3 +44,6 @@ void hostcopy_hold();
 void hostcopy_drop();
 
 }  // namespace dsgdpp
+
+// Bytes that have gone through pieces so far in this process, either way (for tests).
+extern "C" uint64_t dsgdpp_staged_bytes();
