@@ -235,7 +235,8 @@ int mlp_input_count() { return kIn; }
 namespace {
 
 // Samples per CTA: one each while they fit the GPU at a time, then four at a
-// time on at most one CTA per SM.
+// time on at most one CTA per SM (of a B200: the split also says which sums are
+// FP64, so it does not depend on the device).
 MlpGrid mlp_grid(int batch) {
   constexpr int kSMs = 148;
   if (batch <= kSMs) return MlpGrid{1, 1, batch};

@@ -69,3 +69,26 @@ def test_batches_that_fill_and_leave_samples_in_the_last_block(batch):
     moved = net.params - before
     clear = np.abs(g) > 1e-4
     np.testing.assert_allclose(moved[clear], -1e-3 * np.sign(g[clear]), rtol=1e-2)
+
+
+@pytest.mark.parametrize("batch", [1, 3, 148, 149, 592, 1190])
+def test_outputs_are_fp64_sums_rounded_once(batch):
+    # an output of at most 1 rounds by up to 3e-8; FP32 sums of its 64 terms err
+    # by more than 1e-7 in some samples of the larger batches
+    net, rng = _net(batch + 1)
+    X = rng.normal(0, 1.0, (batch, 16)).astype(np.float32)
+    want, _ = M.forward(net.params, X)
+    np.testing.assert_allclose(net.forward(X), want, rtol=0, atol=6e-8)
+
+
+@pytest.mark.parametrize("batch", [1, 3, 64, 148])
+def test_gradients_of_few_samples_near_their_targets(batch):
+    # targets 1e-4 off the outputs: an output that errs by 1e-7 puts 1e-3 of its
+    # gradient in error, the FP32 operations that follow the outputs some 1e-6
+    net, rng = _net(batch + 2)
+    X = rng.normal(0, 1.0, (batch, 16)).astype(np.float32)
+    y = (M.forward(net.params, X)[1][-1] + 1e-4).astype(np.float32)
+    want, wg = M.loss_and_grad(net.params, X, y)
+    loss, g = net.gradient(X, y)
+    assert loss == pytest.approx(want, rel=1e-5)
+    np.testing.assert_allclose(g, wg, rtol=0, atol=1e-5 * np.max(np.abs(wg)))
