@@ -757,7 +757,8 @@ __global__ void build_segments_kernel(SegBuildArgs a) {
 // Measured per epoch against one warp walking each task's records in order:
 // 1M uniform entries, rank 10, d = 4: 294 -> 4.4 ms; rank 32, d = 8: 232 ->
 // 4.1 ms; 500k Zipf(1.1) entries, rank 10, d = 16: 60 -> 34 ms; rank 128,
-// d = 8: 455 -> 67 ms.  With the rows loaded before the slots are known and
+// d = 8: 455 -> 67 ms; one block whose 20,000 records share a column, the other
+// extreme, rank 1 17.5 -> 16.7 ms, 10 22.8 -> 21.0, 128 95.8 -> 39.9.  With the rows loaded before the slots are known and
 // two barriers a round: 4.7 and 36 ms.
 constexpr int kReplayThreads = 512;
 constexpr uint32_t kReplaySlotBits = 11;
@@ -1202,14 +1203,16 @@ cudaError_t replay_launch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
 
 }  // namespace
 
-// Lanes per record by rank, for rows of 4 elements per lane up to rank 32 and
-// of 8 above.  Fewer lanes put more records in hand, which helps blocks
+// Lanes per record by rank, for rows of 2 elements per lane up to rank 8, of 4
+// up to rank 32 and of 8 above.  Fewer lanes put more records in hand, which helps blocks
 // without repeated rows and columns a little and costs where a hot column
 // lets one record run per round (the posts of those that wait queue): rank
 // 10, 1M uniform entries, d = 4 / 500k Zipf(1.1) entries, d = 16, ms per
 // epoch at 8, 4, 2 lanes: 6.3 / 30, 4.4 / 34, 4.1 / 46; rank 32 and 30 at 8
-// and 4 lanes: 4.1 / 43, 3.7 / 60.
+// and 4 lanes: 4.1 / 43, 3.7 / 60.  Two elements per lane take a rank-1 round
+// from 0.94 to 0.84 us, less than a record of the walk in order (0.88).
 cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
+  if (a.r <= 8) return replay_launch<4, 2>(a, s, st);
   if (a.r <= 16) return replay_launch<4, 4>(a, s, st);
   if (a.r <= 32) return replay_launch<8, 4>(a, s, st);
   if (a.r <= 64) return replay_launch<8, 8>(a, s, st);

@@ -827,3 +827,18 @@ def test_sub_epochs_without_entries_keep_the_others_in_order(launch, regularize)
         for a, b in zip(ctx.get_factors(), ref.get_factors()):
             # L2: twelve scales held in FP32, each off by up to 6e-8 of its value
             np.testing.assert_allclose(a, b, rtol=0, atol=5e-6 if regularize == "L2" else 1e-12)
+
+
+@pytest.mark.parametrize("r", [1, 2, 3, 8, 9])
+@pytest.mark.parametrize("kind", ["uniform", "zipf"])
+def test_replay_of_few_elements_per_lane_bit_exact(r, kind):
+    p = _problem(m=300, n=250, nnz=12000, ntest=10, r=r, kind=kind)
+    ref, ctx = _pair(p, r, 2, regularize="L2", regularize_lambda=0.05)
+    with ctx:
+        R = P.Random32(r)
+        for _ in range(2):
+            sched, seeds = P.draw_schedule(R, 2, "COWOR")
+            ctx.epoch_explicit(0.01, sched, seeds)
+            ref.epoch_explicit(0.01, sched, seeds)
+        for a, b in zip(ctx.get_factors(), ref.get_factors()):
+            np.testing.assert_array_equal(a, b)
