@@ -861,10 +861,11 @@ __global__ void __launch_bounds__(kReplayThreads, 1)
     now3 = now3 == 2 ? 0 : now3 + 1;
     if (--rounds_left == 0) {
       // all round numbers used: places count from a new base.  A record in
-      // hand waits for at most K others, of which one runs per round while at
-      // most K are handed out, so its place is within K^2 <= 2^18 of the last
-      // one handed out; what is handed out stays below base + 2^19 + 2^11 K,
-      // within the place bits.
+      // hand waits for at most the K - 1 others, of which the earliest runs in
+      // each round while at most K are handed out, so its place is within K^2
+      // <= 2^14 (K <= 128) of the last one handed out, far less than the 2^19
+      // that the base stays behind; what is handed out until the next base
+      // stays below base + 2^19 + 2^11 K <= base + 2^20, within the place bits.
       rounds_left = (1u << kReplayRoundBits) - 1;
       base = taken > (1u << 19) ? taken - (1u << 19) : 0;
       __syncthreads();  // every group has read its slots

@@ -842,3 +842,27 @@ def test_replay_of_few_elements_per_lane_bit_exact(r, kind):
             ref.epoch_explicit(0.01, sched, seeds)
         for a, b in zip(ctx.get_factors(), ref.get_factors()):
             np.testing.assert_array_equal(a, b)
+
+
+def test_replay_of_a_block_whose_places_count_from_a_new_base():
+    # a round hands out at most 128 records, so the round numbers (2^11) start
+    # over at least once between places 2^19 and 2^19 + 2^18, with all places
+    # after that counted from a base above 0
+    m, n, nnz, r = 3000, 2500, 900_000, 4
+    rng = np.random.default_rng(11)
+    keys = rng.permutation(m * n)[:nnz]
+    rows, cols = (keys // n).astype(np.uint32), (keys % n).astype(np.uint32)
+    vals = rng.standard_normal(nnz)
+    W0, H0 = rng.uniform(-.5, .5, (m, r)), rng.uniform(-.5, .5, (n, r))
+    ref = O.Problem(m, n, r, 1, rows, cols, vals, rows[:5], cols[:5], vals[:5],
+                    method="dsgd")  # one block
+    ref.configure()
+    ref.set_factors(W0, H0)
+    with P.Context(P.Config(m=m, n=n, rank=r, d=1, precision="fp64", exec="replay",
+                            launch="stream", method="dsgd")) as ctx:
+        ctx.set_matrix(P.TRAIN, rows, cols, vals)
+        ctx.set_factors(W0, H0)
+        ctx.epoch_explicit(0.001, [0], [5])
+        ref.epoch_explicit(0.001, [0], [5])
+        for a, b in zip(ctx.get_factors(), ref.get_factors()):
+            np.testing.assert_array_equal(a, b)
