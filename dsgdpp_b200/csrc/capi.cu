@@ -1393,7 +1393,6 @@ int dsgdpp_run(dsgdpp_ctx* c, uint32_t epochs, int decay, double eps0, double de
       check_cuda(cudaEventElapsedTime(&ms, ev.e[from], ev.e[to]), "elapsed");
       return (double)ms * 1e6;
     };
-    if (epochs) draw_epoch(c, sched.data(), seeds.data());
     for (uint32_t e = 0; e < epochs; ++e) {
       auto a = clock::now();
       double eps;
@@ -1409,6 +1408,7 @@ int dsgdpp_run(dsgdpp_ctx* c, uint32_t epochs, int decay, double eps0, double de
       // the epoch and its losses follow one another on the stream and are
       // waited for once; the next epoch's draws (which depend on nothing the
       // epoch computes) are made meanwhile
+      if (e == 0) draw_epoch(c, sched.data(), seeds.data());
       epoch_explicit_impl(c, eps, sched.data(), seeds.data());
       check_cuda(cudaEventRecord(ev.e[0], c->stream), "event");
       enqueue_loss(c, DSGDPP_TRAIN, loss_reg(c), c->h_out);
