@@ -185,8 +185,7 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
               // whole words past the rank, and the upper half of one that ends it
               const uint32_t z = z_last + k * (4 / (uint32_t)sizeof(T));
               const uint32_t keep = z >= r ? 0u : z + 4 / (uint32_t)sizeof(T) > r ? 0xffffu : ~0u;
-              wv[u][c].w[k] &= keep;
-              hv[u][c].w[k] &= keep;
+              wv[u][c].w[k] &= keep;  // H's part reads as finite whatever it holds
             }
           }
           const double before = s;
