@@ -730,11 +730,14 @@ void run_replay_epoch(dsgdpp_ctx* c, double eps, const uint32_t* seeds, uint32_t
   if (s0 == 0) {  // the epoch's inputs, with its first part
   // point orders, one generator per task (mf/sgd/dsgdpp_impl.h:79,112)
   uint64_t total = 0;
+  c->longest_block.resize(d2);
   for (uint32_t s = 0; s < d2; ++s)
     for (uint32_t id = 0; id < d; ++id) {
       c->h_pos_offset[(size_t)s * d + id] = total;
       const uint64_t blk = (uint64_t)id * d2 + c->h_schedule[(size_t)s * d + id];
-      total += M.h_block_ptr[blk + 1] - M.h_block_ptr[blk];
+      const uint64_t n = M.h_block_ptr[blk + 1] - M.h_block_ptr[blk];
+      c->longest_block[s] = std::max(id ? c->longest_block[s] : 0, n);
+      total += n;
     }
   c->h_pos_offset[(size_t)d2 * d] = total;
   if (total > c->positions_cap) {
@@ -792,7 +795,7 @@ void run_replay_epoch(dsgdpp_ctx* c, double eps, const uint32_t* seeds, uint32_t
   a.update = c->cfg.update; a.truncate = c->cfg.truncate;
   a.lambda = c->cfg.update_lambda; a.tmin = c->cfg.truncate_min; a.tmax = c->cfg.truncate_max;
   for (uint32_t s = s0; s < s1; ++s) {
-    check_cuda(launch_replay_subepoch(a, s, st), "replay_subepoch");
+    check_cuda(launch_replay_subepoch(a, s, c->longest_block[s], c->num_sms, st), "replay_subepoch");
     // the W row blocks of the tasks run here
     double* w0 = a.W + c->off1[c->task_lo] * c->rp;
     const uint64_t wrows = c->off1[c->task_hi] - c->off1[c->task_lo];

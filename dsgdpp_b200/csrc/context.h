@@ -117,6 +117,7 @@ struct dsgdpp_ctx {
   uint32_t* h_positions = nullptr;
   uint32_t* d_positions = nullptr;
   uint64_t positions_cap = 0;
+  std::vector<uint64_t> longest_block;  // of each sub-epoch of a replay epoch
   uint64_t* h_pos_offset = nullptr;
   uint64_t* d_pos_offset = nullptr;
   uint8_t* h_mask = nullptr;  // [2d][2d]

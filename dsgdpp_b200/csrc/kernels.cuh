@@ -128,7 +128,9 @@ int hogwild_ctas_per_sm(int precision, uint32_t lanes, uint32_t vecs, bool atomi
 cudaError_t launch_hogwild_epoch(int precision, uint32_t lanes, uint32_t vecs, const HogwildArgs& a,
                                  const EpochDeps& dp, uint32_t grid, cudaStream_t st);
 int hogwild_epoch_ctas_per_sm(int precision, uint32_t lanes, uint32_t vecs, uint32_t nsub);
-cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, cudaStream_t st);
+// longest: records of the sub-epoch's largest block.
+cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, uint64_t longest, int sms,
+                                   cudaStream_t st);
 // RegularizeL2 after sub-epoch s, exactly as the reference (all W, stratum H)
 cudaError_t launch_regularize_exact(double* W, double* H, uint64_t m, uint64_t n, uint32_t rp,
                                     uint32_t r, const uint64_t* off2, const uint8_t* mask,

@@ -12,9 +12,10 @@
 //    the H column.  Within a block updates run concurrently (Hogwild).
 //  * replay_subepoch: the deterministic FP64 mode.  One CTA per task runs its
 //    block with the results of the reference's exact point order, records
-//    without a common row or column together, and repeats every floating-point
-//    operation of the reference in the same order, without FMA contraction, so
-//    the result matches the CPU restatement bit for bit.
+//    without a common row or column together (replay_walk: blocks of a few
+//    records one by one), and repeats every floating-point operation of the
+//    reference in the same order, without FMA contraction, so the result matches
+//    the CPU restatement bit for bit.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -776,6 +777,80 @@ constexpr size_t replay_smem() {
   return sizeof(ReplayRec) * 8 * (kReplayThreads / G) + 4 * sizeof(uint32_t) * kReplaySlots;
 }
 
+// wh = sum_z w[z] h[z] in z order; every lane of a group has the same sum.
+template <int G, int KP>
+__device__ __forceinline__ double replay_dot(const double (&wz)[KP], const double (&hz)[KP],
+                                             uint32_t r) {
+  double pz[KP];
+#pragma unroll
+  for (int k = 0; k < KP; ++k) pz[k] = __dmul_rn(wz[k], hz[k]);
+  double wh = 0;
+#pragma unroll
+  for (int v = 0; v < KP / 2; ++v) {
+    const uint32_t z0 = 2 * G * v;
+    if (z0 >= r) break;
+    if (z0 + 2 * G <= r) {
+#pragma unroll
+      for (int l = 0; l < G; ++l) {
+        wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
+        wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v + 1], l, G));
+      }
+    } else {
+      for (uint32_t l = 0; z0 + 2 * l < r; ++l) {
+        wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
+        const double odd = __shfl_sync(kFullMask, pz[2 * v + 1], l, G);
+        if (z0 + 2 * l + 1 < r) wh = __dadd_rn(wh, odd);
+      }
+    }
+  }
+  return wh;
+}
+
+// The update of one record from its rows' values wz, hz; lane gl of the group
+// writes its elements.
+template <int G, int KP>
+__device__ __forceinline__ void replay_update(const ReplayArgs& a, double* w, double* h,
+                                              const double (&wz)[KP], const double (&hz)[KP],
+                                              uint32_t gl, double x, double wh, double eps,
+                                              double f3, double f4) {
+  const uint32_t r = a.r;
+  // f1 = eps * -2. * (x - wh); f2 = eps * 2. * lambda
+  const double f1 = __dmul_rn(__dmul_rn(eps, -2.0), __dsub_rn(x, wh));
+  const double f2 = __dmul_rn(__dmul_rn(eps, 2.0), a.lambda);
+#pragma unroll
+  for (int v = 0; v < KP / 2; ++v) {
+    const uint32_t z = 2 * (gl + G * v);
+    if (z >= r) continue;
+    double nw[2], nh[2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const double t = wz[2 * v + b], u = hz[2 * v + b];
+      if (a.update == kUpdNzsl) {
+        nw[b] = __dsub_rn(t, __dmul_rn(f1, u));
+        nh[b] = __dsub_rn(u, __dmul_rn(f1, t));
+      } else if (a.update == kUpdNzslL2) {
+        nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(__dmul_rn(f2, t), f3)));
+        nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(__dmul_rn(f2, u), f4)));
+      } else {
+        nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(f2, t)));
+        nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(f2, u)));
+      }
+      if (a.truncate) {
+        if (nw[b] <= a.tmin) nw[b] = __dadd_rn(a.tmin, eps);
+        else if (nw[b] >= a.tmax) nw[b] = __dsub_rn(a.tmax, eps);
+        if (nh[b] <= a.tmin) nh[b] = __dadd_rn(a.tmin, eps);
+        else if (nh[b] >= a.tmax) nh[b] = __dsub_rn(a.tmax, eps);
+      }
+    }
+    if (z + 1 >= r) {  // the padding of an odd rank stays zero
+      nw[1] = 0;
+      nh[1] = 0;
+    }
+    *reinterpret_cast<double2*>(w + z) = make_double2(nw[0], nw[1]);
+    *reinterpret_cast<double2*>(h + z) = make_double2(nh[0], nh[1]);
+  }
+}
+
 // G lanes per record, KP elements of each row per lane (as KP / 2 vectors:
 // element e of vector v of lane l is z = 2 (l + G v) + e); r <= G * KP.
 template <int G, int KP>
@@ -796,9 +871,6 @@ __global__ void __launch_bounds__(kReplayThreads, 1)
   if (n == 0) return;
   const uint32_t* pos = a.positions + a.pos_offset[(size_t)s * d + id];
   const double eps = a.params->eps;
-  // f1 = eps * -2. * (x - wh); f2 = eps * 2. * lambda
-  const double em2 = __dmul_rn(eps, -2.0);
-  const double f2 = __dmul_rn(__dmul_rn(eps, 2.0), a.lambda);
   const bool counts = a.update == kUpdNzslL2;
 
   for (uint32_t k = tid; k < 4 * kReplaySlots; k += kReplayThreads) slots[k] = 0xffffffffu;
@@ -916,64 +988,63 @@ __global__ void __launch_bounds__(kReplayThreads, 1)
 
     // 4. the update
     if (any_go) {
-      double pz[KP];
-#pragma unroll
-      for (int k = 0; k < KP; ++k) pz[k] = __dmul_rn(wz[k], hz[k]);
-      // wh = sum_z w[z] h[z] in z order (every lane of a group has the same sum)
-      double wh = 0;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const uint32_t z0 = 2 * G * v;
-        if (z0 >= r) break;
-        if (z0 + 2 * G <= r) {
-#pragma unroll
-          for (int l = 0; l < G; ++l) {
-            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
-            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v + 1], l, G));
-          }
-        } else {
-          for (uint32_t l = 0; z0 + 2 * l < r; ++l) {
-            wh = __dadd_rn(wh, __shfl_sync(kFullMask, pz[2 * v], l, G));
-            const double odd = __shfl_sync(kFullMask, pz[2 * v + 1], l, G);
-            if (z0 + 2 * l + 1 < r) wh = __dadd_rn(wh, odd);
-          }
-        }
+      const double wh = replay_dot<G, KP>(wz, hz, r);
+      if (go) replay_update<G, KP>(a, w, h, wz, hz, gl, x, wh, eps, f3, f4);
+    }
+  }
+}
+
+// The records of a task in order, one after the other, a warp per task: for
+// sub-epochs of blocks of a few records, where a CTA's tables and loads ahead
+// are most of its time.  32 records' coordinates are loaded at once; a lane
+// reads back only the elements it writes itself, so rows are seen in program
+// order.
+template <int KP>
+__global__ void __launch_bounds__(128) replay_walk_kernel(ReplayArgs a, uint32_t s) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (id >= a.d) return;
+  const uint64_t blk = (uint64_t)id * a.nb2 + a.schedule[(size_t)s * a.d + id];
+  const uint64_t rb = a.block_ptr[blk];
+  const uint32_t n = (uint32_t)(a.block_ptr[blk + 1] - rb);
+  if (n == 0) return;
+  const uint32_t* pos = a.positions + a.pos_offset[(size_t)s * a.d + id];
+  const double eps = a.params->eps;
+  const bool counts = a.update == kUpdNzslL2;
+  for (uint32_t q0 = 0; q0 < n; q0 += 32) {
+    const uint32_t nrec = min(32u, n - q0);
+    ReplayRec e{};
+    if (lane < nrec) {
+      const uint64_t rec = rb + pos[q0 + lane];
+      e.i = a.row[rec];
+      e.j = a.col[rec];
+      e.x = a.val[rec];
+      if (counts) {
+        e.f3 = a.inv1[e.i];
+        e.f4 = a.inv2[e.j];
       }
-      if (go) {
-        const double f1 = __dmul_rn(em2, __dsub_rn(x, wh));
+    }
+    for (uint32_t t = 0; t < nrec; ++t) {
+      double* w = a.W + (size_t)__shfl_sync(kFullMask, e.i, t) * a.rp;
+      double* h = a.H + (size_t)__shfl_sync(kFullMask, e.j, t) * a.rp;
+      const double x = __shfl_sync(kFullMask, e.x, t);
+      const double f3 = __shfl_sync(kFullMask, e.f3, t), f4 = __shfl_sync(kFullMask, e.f4, t);
+      double wz[KP], hz[KP];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          const uint32_t z = 2 * (gl + G * v);
-          if (z >= r) continue;
-          double nw[2], nh[2];
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const double t = wz[2 * v + b], u = hz[2 * v + b];
-            if (a.update == kUpdNzsl) {
-              nw[b] = __dsub_rn(t, __dmul_rn(f1, u));
-              nh[b] = __dsub_rn(u, __dmul_rn(f1, t));
-            } else if (a.update == kUpdNzslL2) {
-              nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(__dmul_rn(f2, t), f3)));
-              nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(__dmul_rn(f2, u), f4)));
-            } else {
-              nw[b] = __dsub_rn(t, __dadd_rn(__dmul_rn(f1, u), __dmul_rn(f2, t)));
-              nh[b] = __dsub_rn(u, __dadd_rn(__dmul_rn(f1, t), __dmul_rn(f2, u)));
-            }
-            if (a.truncate) {
-              if (nw[b] <= a.tmin) nw[b] = __dadd_rn(a.tmin, eps);
-              else if (nw[b] >= a.tmax) nw[b] = __dsub_rn(a.tmax, eps);
-              if (nh[b] <= a.tmin) nh[b] = __dadd_rn(a.tmin, eps);
-              else if (nh[b] >= a.tmax) nh[b] = __dsub_rn(a.tmax, eps);
-            }
-          }
-          if (z + 1 >= r) {  // the padding of an odd rank stays zero
-            nw[1] = 0;
-            nh[1] = 0;
-          }
-          *reinterpret_cast<double2*>(w + z) = make_double2(nw[0], nw[1]);
-          *reinterpret_cast<double2*>(h + z) = make_double2(nh[0], nh[1]);
+      for (int v = 0; v < KP / 2; ++v) {
+        const uint32_t z = 2 * (lane + 32 * v);
+        double2 tw = make_double2(0, 0), th = make_double2(0, 0);
+        if (z < a.rp) {
+          tw = *reinterpret_cast<const double2*>(w + z);
+          th = *reinterpret_cast<const double2*>(h + z);
         }
+        wz[2 * v] = tw.x;
+        wz[2 * v + 1] = tw.y;
+        hz[2 * v] = th.x;
+        hz[2 * v + 1] = th.y;
       }
+      const double wh = replay_dot<32, KP>(wz, hz, a.r);
+      replay_update<32, KP>(a, w, h, wz, hz, lane, x, wh, eps, f3, f4);
     }
   }
 }
@@ -1212,7 +1283,24 @@ cudaError_t replay_launch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
 // epoch at 8, 4, 2 lanes: 6.3 / 30, 4.4 / 34, 4.1 / 46; rank 32 and 30 at 8
 // and 4 lanes: 4.1 / 43, 3.7 / 60.  Two elements per lane take a rank-1 round
 // from 0.94 to 0.84 us, less than a record of the walk in order (0.88).
-cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, cudaStream_t st) {
+//
+// Blocks of few records are walked: the rounds take 10.5 us for a sub-epoch of
+// any few records and 5 us more per further wave (one CTA runs per SM), the
+// walk 5.5 us and, per record of the largest block, 0.45 us at rank 4, 0.65 at
+// 10, 1.0 at 32, 1.1 at 64, 2.2 at 200.  us per sub-epoch, rounds / walk: rank
+// 10, d = 64, largest block of 7 records 10.5 / 9.9, of 12 11.5 / 14.9; d =
+// 1024, 13 records 55 / 29; rank 64, d = 1024, 26 records 88 / 50.
+cudaError_t launch_replay_subepoch(const ReplayArgs& a, uint32_t s, uint64_t longest, int sms,
+                                   cudaStream_t st) {
+  const uint32_t waves = (a.d + sms - 1) / sms;
+  if (longest * (45 + a.r) <= 500 * (uint64_t)waves) {
+    const uint32_t ctas = (a.d + 3) / 4;
+    if (a.r <= 64) replay_walk_kernel<2><<<ctas, 128, 0, st>>>(a, s);
+    else if (a.r <= 128) replay_walk_kernel<4><<<ctas, 128, 0, st>>>(a, s);
+    else if (a.r <= 256) replay_walk_kernel<8><<<ctas, 128, 0, st>>>(a, s);
+    else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+  }
   if (a.r <= 8) return replay_launch<4, 2>(a, s, st);
   if (a.r <= 16) return replay_launch<4, 4>(a, s, st);
   if (a.r <= 32) return replay_launch<8, 4>(a, s, st);

@@ -866,3 +866,21 @@ def test_replay_of_a_block_whose_places_count_from_a_new_base():
         ref.epoch_explicit(0.001, [0], [5])
         for a, b in zip(ctx.get_factors(), ref.get_factors()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("r", [1, 10, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("d,nnz", [(1, 1), (1, 40), (20, 900), (160, 6000)])
+@pytest.mark.parametrize("update,truncate", [("Nzsl", None), ("Nzsl_L2", None),
+                                             ("Nzsl_Nzl2", (-0.4, 0.4))])
+def test_replay_of_blocks_of_few_records_bit_exact(r, d, nnz, update, truncate):
+    # from one record to some ten a block, walked or run in rounds by the rank
+    p = _problem(m=500, n=400, nnz=nnz, ntest=10, r=r)
+    ref, ctx = _pair(p, r, d, update=update, update_lambda=0.5, truncate=truncate)
+    with ctx:
+        R = P.Random32(r)
+        for _ in range(2):
+            sched, seeds = P.draw_schedule(R, d, "COWOR")
+            ctx.epoch_explicit(0.02, sched, seeds)
+            ref.epoch_explicit(0.02, sched, seeds)
+        for a, b in zip(ctx.get_factors(), ref.get_factors()):
+            np.testing.assert_array_equal(a, b)
