@@ -18,8 +18,10 @@ struct dsgdpp_mlp {
   float* m = nullptr;  // Adam moments
   float* v = nullptr;
   float* partials = nullptr;  // rows of partial gradients (grown on demand)
-  // pinned host memory that the kernels read and write: a batch's inputs,
-  // targets and outputs (grown on demand), the gradient and the loss
+  // pinned host memory that the kernels read and write, in one block (grown on
+  // demand; made for kFirstBatch samples): the gradient and the loss, a batch's
+  // inputs, targets and outputs
+  float* pinned = nullptr;
   float* X = nullptr;
   float* Y = nullptr;
   float* out = nullptr;
@@ -34,17 +36,22 @@ namespace {
 
 bool ok(cudaError_t e) { return e == cudaSuccess; }
 
+// a controller's decision is one sample, its training batch 256
+constexpr int kFirstBatch = 256;
+
 int grow(dsgdpp_mlp* n, int batch) {
   if (batch <= n->cap) return DSGDPP_OK;
-  for (float** p : {&n->X, &n->Y, &n->out}) {
-    cudaFreeHost(*p);
-    *p = nullptr;
-  }
+  cudaFreeHost(n->pinned);
+  n->pinned = nullptr;
   n->cap = 0;
-  if (!ok(cudaMallocHost(&n->X, (size_t)batch * mlp_input_count() * 4)) ||
-      !ok(cudaMallocHost(&n->Y, (size_t)batch * 4)) ||
-      !ok(cudaMallocHost(&n->out, (size_t)batch * 4)))
+  const size_t np = mlp_param_count() + 1, in = mlp_input_count();
+  if (!ok(cudaMallocHost(&n->pinned, (np + (size_t)batch * (in + 2)) * 4)))
     return DSGDPP_E_NOMEM;
+  n->grad = n->pinned;
+  n->loss = n->grad + np - 1;
+  n->X = n->grad + np;
+  n->Y = n->X + (size_t)batch * in;
+  n->out = n->Y + batch;
   n->cap = batch;
   return DSGDPP_OK;
 }
@@ -93,8 +100,7 @@ int dsgdpp_mlp_create(int device, uint64_t seed, dsgdpp_mlp** out) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess ||
       !ok(cudaMalloc(&n->P, np * 4)) || !ok(cudaMalloc(&n->m, np * 4)) ||
-      !ok(cudaMalloc(&n->v, np * 4)) || !ok(cudaMallocHost(&n->grad, np * 4)) ||
-      !ok(cudaMallocHost(&n->loss, 4))) {
+      !ok(cudaMalloc(&n->v, np * 4)) || grow(n, kFirstBatch) != DSGDPP_OK) {
     dsgdpp_mlp_destroy(n);
     return DSGDPP_E_CUDA;
   }
@@ -122,7 +128,7 @@ void dsgdpp_mlp_destroy(dsgdpp_mlp* n) {
   cudaSetDevice(n->device);
   if (n->stream) cudaStreamSynchronize(n->stream);
   for (float* p : {n->P, n->m, n->v, n->partials}) cudaFree(p);
-  for (float* p : {n->X, n->Y, n->out, n->grad, n->loss}) cudaFreeHost(p);
+  cudaFreeHost(n->pinned);
   if (n->stream) cudaStreamDestroy(n->stream);
   delete n;
 }
