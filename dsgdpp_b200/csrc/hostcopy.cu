@@ -14,7 +14,12 @@ namespace {
 // 32 / 75 ms through the driver, 8.6 / 16 ms in pieces of 1 MB, 12.5 / 20 ms in
 // pieces of 512 KB.
 constexpr size_t kPiece = 1 << 20;
-constexpr size_t kDirect = 2 << 20;  // below this the driver's own path is as fast
+// Smaller arrays go the driver's way, where making the threads takes longer than
+// they save.  us in / back, direct against pieces: 2.1 MB 152 / 182 against 240 /
+// 479, 4 MB 270 / 320 against 265 / 590, 8 MB 475 / 590 against 473 / 600, 16 MB
+// 910 / 1230 against 660 / 1000.  (Runs of the quick start, whose factors are
+// two arrays of 8 MB, take 5.4 ms with pieces and 6.8 without.)
+constexpr size_t kDirect = 6 << 20;
 constexpr unsigned kThreads = 8;
 // One slab serves one copy.  Page-locking it costs some 7 ms, what the pieces
 // save on about 90 MB, so the first is made once some of that order has been

@@ -2,7 +2,7 @@
 //
 // Arrays that arrive from a file reader or numpy are pageable: the driver
 // copies them through one small page-locked buffer on one core, and the first
-// touch of a result array faults its pages one by one.  Here arrays of a few MB
+// touch of a result array faults its pages one by one.  Here arrays of some MB
 // and up go through page-locked pieces filled (or emptied) by several threads
 // while the previous pieces travel.  Page-locked arrays are copied directly.
 #pragma once

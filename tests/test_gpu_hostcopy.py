@@ -42,7 +42,7 @@ def pieces():
 
 # rows of W of 8 bytes: the bytes of W in 8ths
 @pytest.mark.parametrize("m,staged", [
-    (2 * MB // 8 - 1, False), (2 * MB // 8, True), (2 * MB // 8 + 1, True), (3 * MB // 8, True),
+    (6 * MB // 8 - 1, False), (6 * MB // 8, True), (6 * MB // 8 + 1, True), (7 * MB // 8, True),
     (16 * MB // 8, True), (17 * MB // 8 - 1, True), (33 * MB // 8 + 5, True)])
 def test_factors_of_every_split_into_pieces(pieces, m, staged):
     rng = np.random.default_rng(m)
@@ -60,14 +60,14 @@ def test_factors_of_every_split_into_pieces(pieces, m, staged):
             np.testing.assert_array_equal(H, H0)
 
 
-@pytest.mark.parametrize("nnz", [262_143, 262_145, 524_289, 1_300_001])
+@pytest.mark.parametrize("nnz", [786_431, 786_433, 1_572_865, 2_000_003])
 def test_matrix_through_pieces_and_page_locked(pieces, nnz):
     rng = np.random.default_rng(nnz)
     rows = rng.integers(0, 5000, nnz).astype(np.uint32)  # some pairs repeat: values are summed
     cols = rng.integers(0, 4000, nnz).astype(np.uint32)
     vals = rng.standard_normal(nnz)
     W0, H0 = rng.standard_normal((5000, 4)), rng.standard_normal((4000, 4))
-    sizes = [b for b in (4 * nnz, 4 * nnz, 8 * nnz) if b >= 2 * MB]
+    sizes = [b for b in (4 * nnz, 4 * nnz, 8 * nnz) if b >= 6 * MB]
     got = []
     for give in (np.copy, _lock):
         with P.Context(P.Config(m=5000, n=4000, rank=4, d=3, precision="fp64")) as ctx:
