@@ -183,7 +183,8 @@ void create_impl(dsgdpp_ctx* c, const dsgdpp_config* cfg) {
   check_cuda(cudaMalloc(&c->inv1, cfg->m * cs), "inv1");
   check_cuda(cudaMalloc(&c->inv2, cfg->n * cs), "inv2");
   c->h_schedule = halloc<uint32_t>((size_t)d2 * d, "schedule");
-  c->d_schedule = dalloc<uint32_t>((size_t)d2 * d, "schedule");
+  if (cfg->exec == DSGDPP_EXEC_REPLAY)  // a Hogwild epoch reads h_schedule
+    c->d_schedule = dalloc<uint32_t>((size_t)d2 * d, "schedule");
   c->h_params = halloc<EpochParams>(1, "params");
   c->d_params = dalloc<EpochParams>(1, "params");
   c->h_sigma = halloc<float>((size_t)d2 * d * 3, "sigma");
