@@ -120,13 +120,21 @@ __device__ __forceinline__ uint32_t elem_bits(const Words<N>& v, int e) {
 // at BF16 rank 32; 32 spill, or halve the warps)
 constexpr int kLossWords = 16;
 // BF16 rows of 32 lanes with four vectors (ranks from 769 that fill no 32-byte
-// vector) take 8, and test for a ragged rank at run time: the sums of 32 lanes
-// leave no registers for more, and the test keeps the unpacking of a row's last
-// vector behind that of the others.  2M entries, 16 words / 8 / 8 and the test:
-// rank 776 1063 / - / 971 us, 1000 1110 / 1144 / 975 (16-byte loads, a
-// butterfly per round: 997).  FP32 is slower so (rank 508: 473 -> 709).
+// vector) take 8, and test for a ragged rank at run time (below) whether it is
+// or not: the sums of 32 lanes leave no registers for more.  2M entries, 16
+// words / 8 / 8 and the test: rank 776 1063 / - / 971 us, 1000 1110 / 1144 / 975
+// (16-byte loads, a butterfly per round: 997).  FP32 is slower so (rank 508: 473
+// -> 709).
 template <typename T, int L, int V>
 constexpr bool kTight = sizeof(T) == 2 && L == 32 && V == 4;
+// From 8 lanes on the masked instances test for a ragged rank at run time too.
+// It always is, but the branch keeps the unpacking and masking of a row's last
+// vector behind that of the others, out of the registers that the sums need.
+// 2M entries, us, masked at once / behind the test: FP32 rank 130 225 / 197, 250
+// 390 / 246, 258 470 / 393, 450 816 / 500, 511 597 / 490; BF16 rank 599 707 / 633,
+// 740 735 / 642 (260 306 / 320).
+template <typename T, int L, int V, bool MASK>
+constexpr bool kLateMask = kTight<T, L, V> || (MASK && L >= 8);
 
 // The squared error of 32 entries (nrec of them exist; the others name rows
 // that an entry names: no other row of W or H need be memory of the caller's),
@@ -179,7 +187,7 @@ __device__ __forceinline__ double squares32(uint32_t my_row, uint32_t my_col, fl
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (v0 + c >= V) continue;
-          if ((kTight<T, L, V> ? r % EPV != 0 : MASK) && v0 + c == V - 1) {
+          if ((kLateMask<T, L, V, MASK> ? r % EPV != 0 : MASK) && v0 + c == V - 1) {
 #pragma unroll
             for (int k = 0; k < N; ++k) {
               // whole words past the rank, and the upper half of one that ends it

@@ -884,3 +884,8 @@ def test_replay_of_blocks_of_few_records_bit_exact(r, d, nnz, update, truncate):
             ref.epoch_explicit(0.02, sched, seeds)
         for a, b in zip(ctx.get_factors(), ref.get_factors()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("r", [133, 245, 260, 500, 515, 773, 270, 510, 700, 1023])
+def test_losses_of_bf16_ranks_that_end_inside_a_vector_of_eight_lanes_and_more(r):
+    test_losses_and_norms_of_every_row_mapping("bf16", r, 4129)

@@ -151,3 +151,10 @@ def test_noalloc_calls_of_any_rank_are_captured_after_the_first_call():
     torch.cuda.synchronize()
     want.append(_call(torch, *ids, v, W, H, 200, 200))
     assert out.tolist() == want
+
+
+@pytest.mark.parametrize("r,ld", [(66, 68), (98, 100), (130, 132), (250, 252), (258, 260),
+                                  (378, 380), (450, 452), (135, 136), (253, 256), (381, 384),
+                                  (511, 512)])
+def test_noalloc_masks_the_padding_in_every_mapping_of_eight_lanes_and_more(r, ld):
+    test_noalloc_leaves_padding_and_alignment_to_the_caller(r, ld, 0)
