@@ -84,8 +84,8 @@ __device__ __forceinline__ double f32_scaled(uint32_t b) {
 // four times the lookups.
 //
 // Bound: no single unit -- on 20M Zipf(1.1) entries at rank 32 the L1 data
-// path is 68% busy, instruction issue 53%, the conversion unit and the integer
-// pipe 49%.  Measured there against 2 lanes with four 16-byte vectors, a full
+// path is 69% busy, instruction issue 51%, the conversion unit 48% and the
+// integer pipe 47%.  Measured there against 2 lanes with four 16-byte vectors, a full
 // butterfly per round and zero-filled, predicated loads (ms per loss without
 // factor terms): FP32 rank 10 0.40 -> 0.22, 16 0.33 -> 0.20, 32 0.45 -> 0.31,
 // 50 0.75 -> 0.61, 64 0.73 -> 0.55, 128 1.47 -> 1.05; BF16 rank 32 0.39 ->

@@ -43,6 +43,7 @@ def main():
             ctx.set_factors(data["W0"], data["H0"])
             ctx.seed(args.seed)
             tr = ctx.run(args.epochs, args.decay, args.eps)
+        # time_epoch: the wall time of an epoch without its losses' device time
         out[prec] = {"test_rmse": [math.sqrt(r["test_loss"] / ntest) for r in tr],
                      "epoch_ms_median": float(np.median([r["time_epoch"] for r in tr[1:]]) / 1e6)}
     ref = out["fp64"]["test_rmse"]
